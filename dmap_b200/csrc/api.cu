@@ -328,11 +328,8 @@ static void place_instances(std::vector<TriDev> &t64, std::vector<TriDev32> &t32
         }
         for (int a = 0; a < 3; ++a) {
             S.q0[a] = q2[a];
-            S.q0f[a] = (float)q2[a];
-            for (int b = 0; b < 3; ++b) {
+            for (int b = 0; b < 3; ++b)
                 S.A[a][b] = A2[a][b];
-                S.Af[a][b] = (float)A2[a][b];
-            }
         }
     }
 }
@@ -441,6 +438,8 @@ static dmap_status scene_create(dmap_context *ctx, dmap_asset *const *assets, in
     s->tris_host.resize(n_tri);
     if ((e = cudaMemcpy(s->tris_host.data(), s->tris_dev, sizeof(TriDev) * n_tri, cudaMemcpyDeviceToHost)))
         return cleanup(cuda_fail(ctx, e, "dmap_scene_create: readback"));
+    for (const TriDev &T : s->tris_host)
+        s->deep |= T.root_level > 15 ? 1 : 0;
     cudaFree(tris_dev);
     cudaFree(ta_dev);
     tris_dev = nullptr;
@@ -686,6 +685,7 @@ dmap_status dmapi::check_query(dmap_scene *s, dmap_dtype ray_dtype, int64_t n, c
     q.bvh_range = reinterpret_cast<const int4 *>(s->bvh_range_dev);
     q.inst_xf = s->inst_dev;
     q.bvh_n_nodes = s->bvh_n_nodes;
+    q.deep = s->deep;
     apply_filter(s, q);
     return DMAP_OK;
 }

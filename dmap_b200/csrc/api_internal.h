@@ -81,6 +81,7 @@ struct dmap_scene
     double *inst_dev = nullptr; // non-rigid instances: their transforms (instance.cuh), else null
     int n_inst = 0;
     int bvh_n_nodes = 0;
+    int deep = 0; // a triangle's root level is above 15 (QueryOpts::deep)
     std::vector<TriDev> tris_host;
     bool all_f64 = true;
     // the opacity filter (dmap_scene_set_opacity); op_mask_dev null: none

@@ -56,31 +56,27 @@ struct TriDev
     int inst, inst_pad;
 };
 
-// The FP32 record: the same geometry rounded to float, plus the FP64 frame
-// origin and matrix for the per-ray transform.
-struct TriDev32
+// The FP32 record: what the walk reads, plus the FP64 frame origin and
+// matrix for the per-ray transform. The node test and the domain test read
+// the first 128 bytes (one cache line) as eight 16-byte loads
+// (f32_node.cuh:load_walk).
+struct alignas(128) TriDev32
 {
-    float e1[3], e2[3], m0[3], Mu[3], Mv[3];
-    float q0f[3];
-    float t0[2], t1[2], t2[2];
-    float J[2][2];
-    float Af[3][3];        // to_tangent rounded to nearest
+    // The interpolated normal in tangent space, A N(s,t) = a0 + s au + t av,
+    // per axis (a0, au, av, rowsum), rowsum = sum_j |A_ij| bounding |A n| for
+    // a unit n; |N(s,t)|^2 = qc + 2 s q1 + 2 t q2 + s^2 q11 + 2 s t q12 +
+    // t^2 q22; all rounded from double.
+    float nrm[3][4];
+    float qc, q1, q2, q11, q12, q22;
+    float lo[2], hi[2];    // texture-space box of the domain, outward
     float un[3][2], ud[3]; // domain edges (exact for dyadic texture coordinates)
-    float lo[2], hi[2];
-    float box_lo[3], box_hi[3]; // object AABB widened outward
-    float residual_tol;
-    float newton_tol;      // FP32 acceptance tolerance of the Newton residual
-    float mean_edge;
+    int log2n;             // the asset's pyramid: 2^log2n leaf cells per side
+    const float *pyr32;
     int root_level, n_roots, asset, pad;
     int roots_i[4], roots_j[4];
     double A[3][3];        // to_tangent in double for the ray transform
     double q0[3];
-    // The interpolated normal in tangent space, A N(s,t) = a0 + s au + t av,
-    // and |N(s,t)|^2 = qc + 2 s q1 + 2 t q2 + s^2 q11 + 2 s t q12 + t^2 q22,
-    // rounded from double; rowsum[i] = sum_j |A_ij| bounds |A n| for a unit n.
-    float a0[3], au[3], av[3];
-    float qc, q1, q2, q11, q12, q22;
-    float rowsum[3];
+    float box_lo[3], box_hi[3]; // object AABB widened outward
 };
 
 // Device status word bits (written with atomicOr).

@@ -29,33 +29,65 @@ __device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) 
 
 struct Node32 { float h0, gu, gv, r, mn, mx; };
 
-// TaylorPyramid::node (taylor_pyramid.cpp:259-274) on the FP32 pyramid:
-// wrapped indices (the level's width is a power of two), above the root the
-// root's height range as a min-max node.
-__device__ __forceinline__ Node32 fetch_node(const AssetDev &a, int level, int i, int j)
+// First cell of level l of a pyramid over 2^L x 2^L leaf cells: the sum of
+// 4^(L - m) over m < l, that is 4^(L + 1 - l) (4^l - 1) / 3.
+__device__ __forceinline__ int64_t level_first(int L, int l)
+{
+    return (int64_t)((0x5555555555555555ull & ((1ull << (2 * l)) - 1ull)) << (2 * (L + 1 - l)));
+}
+
+// TaylorPyramid::node (taylor_pyramid.cpp:259-274) on the FP32 pyramid of
+// 2^L x 2^L leaf cells: wrapped indices (the level's width is a power of
+// two), above the root the root's height range as a min-max node.
+__device__ __forceinline__ Node32 fetch_node(const float *pyr32, int L, int level, int i, int j)
 {
     Node32 n;
-    if (level >= a.n_levels) {
-        const float4 *p = reinterpret_cast<const float4 *>(a.pyr32 + 8 * a.level_off[a.n_levels - 1]);
-        float4 q1 = __ldg(p + 1);
-        n.mn = q1.z;
-        n.mx = q1.w;
-        n.h0 = 0.5f * (n.mn + n.mx);
-        n.r = fmaxf(__fsub_ru(n.mx, n.h0), __fsub_ru(n.h0, n.mn));
-        n.gu = n.gv = 0.0f;
-        return n;
-    }
-    int m = a.n_leaf >> level;
-    int ri = i & (m - 1), rj = j & (m - 1);
-    const float4 *p = reinterpret_cast<const float4 *>(a.pyr32 + 8 * (a.level_off[level] + (int64_t)rj * m + ri));
-    float4 q0 = __ldg(p), q1 = __ldg(p + 1);
+    const bool above = level > L;
+    const int lv = above ? L : level;
+    const int m1 = (1 << (L - lv)) - 1;
+    const int64_t at = level_first(L, lv) + (((int64_t)(j & m1)) << (L - lv)) + (i & m1);
+    const float4 *p = reinterpret_cast<const float4 *>(pyr32 + 8 * at);
+    const float4 q0 = __ldg(p), q1 = __ldg(p + 1);
     n.h0 = q0.x;
     n.gu = q0.y;
     n.gv = q0.z;
     n.r = q0.w;
     n.mn = q1.z;
     n.mx = q1.w;
+    if (above) {
+        n.h0 = 0.5f * (n.mn + n.mx);
+        n.r = fmaxf(__fsub_ru(n.mx, n.h0), __fsub_ru(n.h0, n.mn));
+        n.gu = n.gv = 0.0f;
+    }
     return n;
+}
+
+// The first 128 bytes of a triangle's FP32 record, loaded as eight 16-byte
+// words: what the node test and the domain test read.
+struct Walk32
+{
+    float4 n[3]; // per axis: a0, au, av, rowsum
+    float qc, q1, q2, q11, q12, q22;
+    float lox, loy, hix, hiy;
+    float ux[3], uy[3], ud[3];
+    int log2n;
+};
+
+__device__ __forceinline__ Walk32 load_walk(const TriDev32 &T)
+{
+    const float4 *p = reinterpret_cast<const float4 *>(&T);
+    const float4 a = __ldg(p + 3), b = __ldg(p + 4), c = __ldg(p + 5), d = __ldg(p + 6), e = __ldg(p + 7);
+    Walk32 w;
+    w.n[0] = __ldg(p);
+    w.n[1] = __ldg(p + 1);
+    w.n[2] = __ldg(p + 2);
+    w.qc = a.x, w.q1 = a.y, w.q2 = a.z, w.q11 = a.w;
+    w.q12 = b.x, w.q22 = b.y;
+    w.lox = b.z, w.loy = b.w, w.hix = c.x, w.hiy = c.y;
+    w.ux[0] = c.z, w.uy[0] = c.w, w.ux[1] = d.x, w.uy[1] = d.y, w.ux[2] = d.z, w.uy[2] = d.w;
+    w.ud[0] = e.x, w.ud[1] = e.y, w.ud[2] = e.z;
+    w.log2n = __float_as_int(e.w);
+    return w;
 }
 
 // The tangent-space ray (o, d), its reciprocal directions and the widening
@@ -90,15 +122,15 @@ __device__ __forceinline__ void cell_next(Cell32 &c, int si, int sj, int root_le
 
 // classify_square (uv_clip.cpp:27-44) reporting Outside only when the
 // separation exceeds the rounding of the test.
-__device__ __forceinline__ bool square_meets_domain(const TriDev32 &T, float cx, float cy, float s)
+__device__ __forceinline__ bool square_meets_domain(const Walk32 &T, float cx, float cy, float s)
 {
-    if (cx + s <= T.lo[0] || cx - s >= T.hi[0] || cy + s <= T.lo[1] || cy - s >= T.hi[1])
+    if (cx + s <= T.lox || cx - s >= T.hix || cy + s <= T.loy || cy - s >= T.hiy)
         return false;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        float proj = __fmaf_rn(T.un[k][1], cy, T.un[k][0] * cx);
-        float ext = (fabsf(T.un[k][0]) + fabsf(T.un[k][1])) * s;
-        float slack = G * (fabsf(T.un[k][0] * cx) + fabsf(T.un[k][1] * cy) + fabsf(T.ud[k]) + ext);
+        float proj = __fmaf_rn(T.uy[k], cy, T.ux[k] * cx);
+        float ext = (fabsf(T.ux[k]) + fabsf(T.uy[k])) * s;
+        float slack = G * (fabsf(T.ux[k] * cx) + fabsf(T.uy[k] * cy) + fabsf(T.ud[k]) + ext);
         if (proj + ext + slack <= T.ud[k])
             return false;
     }
@@ -137,7 +169,7 @@ __device__ __forceinline__ void clip_axis(float o, float d, float inv, float lo,
 // The range of 1/|N| over the rectangle [cx +- hx] x [cy +- hy], with
 // |N(s,t)|^2 = qc + 2 s q1 + 2 t q2 + s^2 q11 + 2 s t q12 + t^2 q22, as
 // midpoint rm and radius rr; false when |N| may vanish there.
-__device__ __forceinline__ bool inv_norm_range(const TriDev32 &T, float cx, float cy, float hx, float hy, float &rm,
+__device__ __forceinline__ bool inv_norm_range(const Walk32 &T, float cx, float cy, float hx, float hy, float &rm,
                                                float &rr)
 {
     float gs = 2.0f * hx * __fmaf_rn(cy, T.q12, __fmaf_rn(cx, T.q11, T.q1));
@@ -203,14 +235,14 @@ __device__ __forceinline__ void box_axis(float a0, float au, float av, float cx,
 
 // The node test of one cell (node_bounds.cpp:83-211): the box, and at levels
 // <= slab_max_level the slab, both enclosing their double counterparts.
-__device__ __forceinline__ bool node_test32(const TriDev32 &T, const AssetDev &a, const Ray32 &r, int level, int i,
+__device__ __forceinline__ bool node_test32(const Walk32 &T, const float *pyr32, const Ray32 &r, int level, int i,
                                             int j, float t_min, float t_max, int bound, int slab_max_level)
 {
-    Node32 n = fetch_node(a, level, i, j);
-    float w = pow2f(level - (__ffs(a.n_leaf) - 1));
+    Node32 n = fetch_node(pyr32, T.log2n, level, i, j);
+    float w = pow2f(level - T.log2n);
     float u0 = ((float)i + 0.5f) * w, v0 = ((float)j + 0.5f) * w;
-    float rlx = fmaxf((float)i * w, T.lo[0]), rly = fmaxf((float)j * w, T.lo[1]);
-    float rhx = fminf((float)(i + 1) * w, T.hi[0]), rhy = fminf((float)(j + 1) * w, T.hi[1]);
+    float rlx = fmaxf((float)i * w, T.lox), rly = fmaxf((float)j * w, T.loy);
+    float rhx = fminf((float)(i + 1) * w, T.hix), rhy = fminf((float)(j + 1) * w, T.hiy);
     float cx = 0.5f * (rlx + rhx), cy = 0.5f * (rly + rhy);
     float hx = fmaxf(fmaxf(__fsub_ru(rhx, cx), __fsub_ru(cx, rlx)), 0.0f);
     float hy = fmaxf(fmaxf(__fsub_ru(rhy, cy), __fsub_ru(cy, rly)), 0.0f);
@@ -219,11 +251,11 @@ __device__ __forceinline__ bool node_test32(const TriDev32 &T, const AssetDev &a
     float mid = 0.5f * (n.mn + n.mx);
     float hh = fmaxf(__fsub_ru(n.mx, mid), __fsub_ru(mid, n.mn));
     float lx, hx_, ly, hy_, lz, hz, mxl, mxh, myl, myh, mzl, mzh;
-    box_axis(T.a0[0], T.au[0], T.av[0], cx, cy, hx, hy, ok, rm, rr, T.rowsum[0], mid, hh, cx, hx, 0.0f, r.ex, lx,
+    box_axis(T.n[0].x, T.n[0].y, T.n[0].z, cx, cy, hx, hy, ok, rm, rr, T.n[0].w, mid, hh, cx, hx, 0.0f, r.ex, lx,
              hx_, mxl, mxh);
-    box_axis(T.a0[1], T.au[1], T.av[1], cx, cy, hx, hy, ok, rm, rr, T.rowsum[1], mid, hh, cy, 0.0f, hy, r.ey, ly,
+    box_axis(T.n[1].x, T.n[1].y, T.n[1].z, cx, cy, hx, hy, ok, rm, rr, T.n[1].w, mid, hh, cy, 0.0f, hy, r.ey, ly,
              hy_, myl, myh);
-    box_axis(T.a0[2], T.au[2], T.av[2], cx, cy, hx, hy, ok, rm, rr, T.rowsum[2], mid, hh, 0.0f, 0.0f, 0.0f, r.ez,
+    box_axis(T.n[2].x, T.n[2].y, T.n[2].z, cx, cy, hx, hy, ok, rm, rr, T.n[2].w, mid, hh, 0.0f, 0.0f, 0.0f, r.ez,
              lz, hz, mzl, mzh);
     bool read_slab = level <= slab_max_level;
     float b0 = t_min, b1 = t_max;
@@ -293,6 +325,16 @@ __device__ __forceinline__ void load_ray(const R *rays, int64_t k, double *o, do
     dmapdev::sanitize_ray(o, d, t_min, t_max);
 }
 
+// The same for a ray record type chosen at run time (QueryOpts::ray_dtype).
+__device__ __forceinline__ void load_ray(const void *rays, int ray_dtype, int64_t k, double *o, double *d,
+                                         double &t_min, double &t_max)
+{
+    if (ray_dtype == 2)
+        load_ray(static_cast<const double *>(rays), k, o, d, t_min, t_max);
+    else
+        load_ray(static_cast<const float *>(rays), k, o, d, t_min, t_max);
+}
+
 template <typename H, typename Fp>
 __device__ __forceinline__ void store_hit(H *hits, int64_t k, bool found, const d64::hit64 &h, int tri, int flags)
 {
@@ -319,6 +361,16 @@ __device__ __forceinline__ void store_hit(H *hits, int64_t k, bool found, const 
         out.flags = flags;
     }
     hits[k] = out;
+}
+
+// The same for a hit record type chosen at run time (QueryOpts::hit_dtype).
+__device__ __forceinline__ void store_hit(void *hits, int hit_dtype, int64_t k, bool found, const d64::hit64 &h,
+                                          int tri, int flags)
+{
+    if (hit_dtype == 2)
+        store_hit<dmapdev::Hit64, double>(static_cast<dmapdev::Hit64 *>(hits), k, found, h, tri, flags);
+    else
+        store_hit<dmapdev::Hit32, float>(static_cast<dmapdev::Hit32 *>(hits), k, found, h, tri, flags);
 }
 
 // A leaf cell the FP32 walk reached: first the reference's own node test of

@@ -26,6 +26,8 @@ struct QueryOpts
     // runs (at most the n the launch is given, which sizes grids and scratch):
     // stages of a device-driven pipeline pass counts they produced themselves.
     const long long *n_dev = nullptr;
+    // FP32 walk: a triangle's root level is above 15 (wave_walk's DEEP, walk32.cuh)
+    int deep = 0;
     // Scenes of more than 256 triangles: the tree over the triangles' FP32
     // boxes that both candidate orders walk (bvh.cuh gives the layout), bvh_n_nodes
     // inner nodes of 4 float4, 2 float4 per triangle list position.

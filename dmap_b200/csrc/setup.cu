@@ -216,31 +216,17 @@ __device__ void setup_one(TriDev &T, const AssetDev &a, unsigned *status)
 __device__ float fdown(double x) { return __double2float_rd(x); }
 __device__ float fup(double x) { return __double2float_ru(x); }
 
-__device__ void derive32(const TriDev &T, TriDev32 &S)
+__device__ void derive32(const TriDev &T, const AssetDev &g, TriDev32 &S)
 {
     for (int a = 0; a < 3; ++a) {
-        S.e1[a] = (float)T.e1[a];
-        S.e2[a] = (float)T.e2[a];
-        S.m0[a] = (float)T.m0[a];
-        S.Mu[a] = (float)T.Mu[a];
-        S.Mv[a] = (float)T.Mv[a];
-        S.q0f[a] = (float)T.q0[a];
         S.q0[a] = T.q0[a];
-        for (int b = 0; b < 3; ++b) {
-            S.Af[a][b] = (float)T.A[a][b];
+        for (int b = 0; b < 3; ++b)
             S.A[a][b] = T.A[a][b];
-        }
         // object AABB widened by a few float ulps of its magnitude
         double pad = 4.0 * 1.1920928955078125e-7 * (1.0 + fmax(fabs(T.box_lo[a]), fabs(T.box_hi[a])));
         S.box_lo[a] = fdown(T.box_lo[a] - pad);
         S.box_hi[a] = fup(T.box_hi[a] + pad);
     }
-    S.t0[0] = (float)T.t0[0], S.t0[1] = (float)T.t0[1];
-    S.t1[0] = (float)T.t1[0], S.t1[1] = (float)T.t1[1];
-    S.t2[0] = (float)T.t2[0], S.t2[1] = (float)T.t2[1];
-    for (int a = 0; a < 2; ++a)
-        for (int b = 0; b < 2; ++b)
-            S.J[a][b] = (float)T.J[a][b];
     for (int k = 0; k < 3; ++k) {
         S.un[k][0] = (float)T.un[k][0];
         S.un[k][1] = (float)T.un[k][1];
@@ -248,9 +234,8 @@ __device__ void derive32(const TriDev &T, TriDev32 &S)
     }
     S.lo[0] = fdown(T.lo[0]), S.lo[1] = fdown(T.lo[1]);
     S.hi[0] = fup(T.hi[0]), S.hi[1] = fup(T.hi[1]);
-    S.residual_tol = (float)T.residual_tol;
-    S.mean_edge = (float)(T.residual_tol * 1e10);
-    S.newton_tol = 0.0f; // set by the FP32 path from the ray scale
+    S.log2n = __ffs(g.n_leaf) - 1;
+    S.pyr32 = g.pyr32;
     S.root_level = T.root_level;
     S.n_roots = T.n_roots;
     S.asset = T.asset;
@@ -262,10 +247,10 @@ __device__ void derive32(const TriDev &T, TriDev32 &S)
     v3 m0 = L3(T.m0), Mu = L3(T.Mu), Mv = L3(T.Mv);
     v3 a0 = mat3mul(T.A, m0), au = mat3mul(T.A, Mu), av = mat3mul(T.A, Mv);
     for (int a = 0; a < 3; ++a) {
-        S.a0[a] = (float)comp(a0, a);
-        S.au[a] = (float)comp(au, a);
-        S.av[a] = (float)comp(av, a);
-        S.rowsum[a] = fup((fabs(T.A[a][0]) + fabs(T.A[a][1])) + fabs(T.A[a][2]));
+        S.nrm[a][0] = (float)comp(a0, a);
+        S.nrm[a][1] = (float)comp(au, a);
+        S.nrm[a][2] = (float)comp(av, a);
+        S.nrm[a][3] = fup((fabs(T.A[a][0]) + fabs(T.A[a][1])) + fabs(T.A[a][2]));
     }
     S.qc = (float)dot3(m0, m0);
     S.q1 = (float)dot3(m0, Mu);
@@ -296,7 +281,7 @@ __global__ void setup_kernel(const double *__restrict__ tris, int stride, const 
     setup_one(T, assets[T.asset], status);
     out[k] = T;
     TriDev32 S;
-    derive32(T, S);
+    derive32(T, assets[T.asset], S);
     out32[k] = S;
 }
 

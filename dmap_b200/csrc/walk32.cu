@@ -10,7 +10,6 @@ namespace dmapk
 namespace w32
 {
 
-template <typename R, typename H, typename Fp>
 cudaError_t walk_round(const Args &a, const int *q_in, int round, cudaStream_t stream)
 {
     // scenes of more than 256 triangles take the triangle tree; each
@@ -18,23 +17,23 @@ cudaError_t walk_round(const Args &a, const int *q_in, int round, cudaStream_t s
     // kernel carries one order's candidate code, and scenes of up to 256
     // triangles keep the smaller kernel
     const bool nearest = a.opt.order == 1, tree = a.n_tri > 32 * kMaskWords;
-    const R *rr = static_cast<const R *>(a.rays);
-    H *hh = static_cast<H *>(a.hits);
     RayState *states = static_cast<RayState *>(a.states);
     LeafJob *leaves = static_cast<LeafJob *>(a.leaves);
-#define DMAP_ROUND(ST_, TR_, NR_)                                                                                   \
-    wave_walk<ST_, false, TR_, NR_, R, H, Fp><<<a.grid, 128, 0, stream>>>(a.t32, a.t64, a.n_tri, a.assets, rr, a.n, \
-                                                                          a.opt, hh, ST_ ? a.stats : nullptr,      \
-                                                                          states, q_in, round, leaves, a.counters, \
-                                                                          a.status, a.rerun)
+#define DMAP_ROUND(ST_, TR_, NR_, DP_)                                                                              \
+    wave_walk<ST_, false, TR_, NR_, DP_><<<a.grid, 128, 0, stream>>>(                                     \
+        a.t32, a.t64, a.n_tri, a.assets, a.rays, a.n, a.opt, a.hits, ST_ ? a.stats : nullptr, states, q_in, round, leaves,  \
+        a.counters, a.status, a.rerun)
+#define DMAP_ROUND_DEEP(ST_, TR_, NR_)                                                                              \
+    (ST_ || a.opt.deep ? DMAP_ROUND(ST_, TR_, NR_, true) : DMAP_ROUND(false, TR_, NR_, false))
 #define DMAP_ROUND_MODE(ST_)                                                                                        \
-    (tree ? (nearest ? DMAP_ROUND(ST_, true, true) : DMAP_ROUND(ST_, true, false))                                  \
-          : (nearest ? DMAP_ROUND(ST_, false, true) : DMAP_ROUND(ST_, false, false)))
+    (tree ? (nearest ? DMAP_ROUND_DEEP(ST_, true, true) : DMAP_ROUND_DEEP(ST_, true, false))                        \
+          : (nearest ? DMAP_ROUND_DEEP(ST_, false, true) : DMAP_ROUND_DEEP(ST_, false, false)))
     if (a.stats)
         DMAP_ROUND_MODE(true);
     else
         DMAP_ROUND_MODE(false);
 #undef DMAP_ROUND_MODE
+#undef DMAP_ROUND_DEEP
 #undef DMAP_ROUND
     return cudaGetLastError();
 }
@@ -65,7 +64,7 @@ cudaError_t launch(Args a, const WaveScratch &ws, cudaStream_t stream)
     const int bps = a.opt.blocks_per_sm > 0              ? a.opt.blocks_per_sm
                     : a.n_tri > 32 * kMaskWords ? DMAP_WALK_TREE_MIN_BLOCKS
                                                          : DMAP_WALK_MIN_BLOCKS;
-    const int64_t need = (a.n + 127) / 128;
+    const int64_t need = (a.n + 31) / 32; // four lanes per ray
     a.grid = sm_count() * bps;
     if (need < a.grid)
         a.grid = (int)need;
@@ -77,11 +76,11 @@ cudaError_t launch(Args a, const WaveScratch &ws, cudaStream_t stream)
         const int *q_in = ws.queue[(rd + 1) & 1];
         int *q_out = ws.queue[rd & 1];
         if (rd == rounds) {
-            if ((e = walk_drain<R, H, Fp>(a, q_in, rd, stream)) != cudaSuccess || !a.opt.op_mask)
+            if ((e = walk_drain(a, q_in, rd, stream)) != cudaSuccess || !a.opt.op_mask)
                 return e;
             return simple_rerun<R, H, Fp>(a, stream);
         }
-        if ((e = walk_round<R, H, Fp>(a, q_in, rd, stream)) != cudaSuccess ||
+        if ((e = walk_round(a, q_in, rd, stream)) != cudaSuccess ||
             (e = filter<R>(a, rd, stream)) != cudaSuccess)
             return e;
         e = a.opt.leaf_precision == 1 ? leaf32<R, H, Fp>(a, rd, q_out, stream) // the FP32 certified leaf

@@ -23,9 +23,9 @@
 //    while the others wait (measured 1.6 active threads per warp
 //    instruction on the cube-sphere workload).
 //  - wavefront (default): rounds of two persistent kernels. The walk kernel
-//    keeps every lane on a node test each step: a lane whose ray reaches a
-//    leaf writes a leaf job, parks the ray's walk state and takes the next
-//    ray; the leaf kernel runs the parked leaves, one job per lane, each
+//    gives each ray four lanes, which test the four cells of a sibling group
+//    together: a ray that reaches leaves writes a leaf job, parks its walk
+//    state and its lanes take the next ray; the leaf kernel runs the parked leaves, one job per lane, each
 //    lane taking the next job when its own is done, and queues their rays
 //    to resume. After `rounds` rounds a last walk runs the few
 //    remaining rays with their leaves inline. Every ray still visits its
@@ -88,30 +88,32 @@ constexpr unsigned FULL = 0xffffffffu;
 // order): the rounding to float, at most 2^-24 of each coordinate (2^-22
 // taken), plus the difference of two double evaluations of the transform,
 // a few units of 2^-53 of the sums of the terms' magnitudes (2^-40 taken).
+__device__ __forceinline__ void tangent_row(const TriDev32 &T, int a, const double *o, const double *d, float t_far,
+                                            float &ro, float &rd, float &e)
+{
+    const double A0 = T.A[a][0], A1 = T.A[a][1], A2 = T.A[a][2];
+    double u0 = o[0] - T.q0[0], u1 = o[1] - T.q0[1], u2 = o[2] - T.q0[2];
+    double x = A0 * u0;
+    x = __fma_rn(A1, u1, x);
+    x = __fma_rn(A2, u2, x);
+    double y = __fma_rn(A2, d[2], __fma_rn(A1, d[1], A0 * d[0]));
+    double mx = fabs(A0 * u0) + fabs(A1 * u1) + fabs(A2 * u2);
+    double my = fabs(A0 * d[0]) + fabs(A1 * d[1]) + fabs(A2 * d[2]);
+    ro = (float)x;
+    rd = (float)y;
+    float sum = ru_add(__double2float_ru(mx), ru_mul(t_far, __double2float_ru(my)));
+    e = ru_add(ru_mul(0x1p-22f, ru_add(fabsf(ro), ru_mul(t_far, fabsf(rd)))), ru_mul(0x1p-40f, sum));
+}
+
 __device__ __forceinline__ void tangent_ray(const TriDev32 &T, const double *o, const double *d, float t_far,
                                             Ray32 &r)
 {
-    float ro[3], rd[3], e[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        double u0 = o[0] - T.q0[0], u1 = o[1] - T.q0[1], u2 = o[2] - T.q0[2];
-        double x = u0 * T.A[a][0];
-        x = __fma_rn(T.A[a][1], u1, x);
-        x = __fma_rn(T.A[a][2], u2, x);
-        double y = __fma_rn(T.A[a][2], d[2], __fma_rn(T.A[a][1], d[1], T.A[a][0] * d[0]));
-        double mx = fabs(T.A[a][0] * u0) + fabs(T.A[a][1] * u1) + fabs(T.A[a][2] * u2);
-        double my = fabs(T.A[a][0] * d[0]) + fabs(T.A[a][1] * d[1]) + fabs(T.A[a][2] * d[2]);
-        ro[a] = (float)x;
-        rd[a] = (float)y;
-        float sum = ru_add(__double2float_ru(mx), ru_mul(t_far, __double2float_ru(my)));
-        e[a] = ru_add(ru_mul(0x1p-22f, ru_add(fabsf(ro[a]), ru_mul(t_far, fabsf(rd[a])))), ru_mul(0x1p-40f, sum));
-    }
-    r.ox = ro[0], r.oy = ro[1], r.oz = ro[2];
-    r.dx = rd[0], r.dy = rd[1], r.dz = rd[2];
+    tangent_row(T, 0, o, d, t_far, r.ox, r.dx, r.ex);
+    tangent_row(T, 1, o, d, t_far, r.oy, r.dy, r.ey);
+    tangent_row(T, 2, o, d, t_far, r.oz, r.dz, r.ez);
     r.ix = r.dx != 0.0f ? __frcp_rn(r.dx) : 0.0f;
     r.iy = r.dy != 0.0f ? __frcp_rn(r.dy) : 0.0f;
     r.iz = r.dz != 0.0f ? __frcp_rn(r.dz) : 0.0f;
-    r.ex = e[0], r.ey = e[1], r.ez = e[2];
 }
 
 __device__ __forceinline__ float far_bound(float t1) { return ru_add(ru_mul(t1, 1.0f + 4.0f * G), G); }
@@ -159,7 +161,7 @@ __device__ bool triangle_walk32(const TriDev32 &T, const TriDev &T64, const Asse
     float tmin_f = __double2float_rd(t_min);
     bool found = false;
     int64_t nah = 0, lah = 0;
-    const int log2n = __ffs(g.n_leaf) - 1;
+    const Walk32 W = load_walk(T);
     for (int q = 0; q < T.n_roots; ++q) {
         Cell32 cur = {T.root_level, T.roots_i[q], T.roots_j[q]}, end = cur;
         cell_next(end, si, sj, T.root_level);
@@ -170,8 +172,8 @@ __device__ bool triangle_walk32(const TriDev32 &T, const TriDev &T64, const Asse
                 capped = true;
                 break;
             }
-            float w = pow2f(cur.level - log2n);
-            if (!square_meets_domain(T, ((float)cur.i + 0.5f) * w, ((float)cur.j + 0.5f) * w, 0.5f * w)) {
+            float w = pow2f(cur.level - W.log2n);
+            if (!square_meets_domain(W, ((float)cur.i + 0.5f) * w, ((float)cur.j + 0.5f) * w, 0.5f * w)) {
                 cell_next(cur, si, sj, T.root_level);
                 continue;
             }
@@ -180,7 +182,8 @@ __device__ bool triangle_walk32(const TriDev32 &T, const TriDev &T64, const Asse
                 ++nah;
             }
             float tmax_f = __double2float_ru(t_max);
-            if (!node_test32(T, g, r, cur.level, cur.i, cur.j, tmin_f, tmax_f, opt.bound, opt.slab_max_level)) {
+            if (!node_test32(W, T.pyr32, r, cur.level, cur.i, cur.j, tmin_f, tmax_f, opt.bound,
+                             opt.slab_max_level)) {
                 cell_next(cur, si, sj, T.root_level);
                 continue;
             }
@@ -331,18 +334,78 @@ __global__ void __launch_bounds__(128) walk32_simple(const TriDev32 *__restrict_
 
 // ---- wavefront schedule ---------------------------------------------------------
 
+// One bit per cell of a stackless walk's open sibling groups: child k of the
+// group at level l (k counts the siblings in the ray's visiting order) is bit
+// 4 l + k, so the lowest bit is the next cell of the depth-first order. The
+// walk has one open group per level, and the roots are the group of the root
+// level. 64 bits hold root levels up to 15; scenes with a higher one (repeat
+// charts over many tiles, maps beyond 32768 texels) take DEEP, up to 31.
+template <bool DEEP>
+struct CellBits
+{
+    unsigned long long lo, hi;
+    __device__ __forceinline__ bool any() const { return DEEP ? (lo | hi) != 0ull : lo != 0ull; }
+    __device__ __forceinline__ int first() const
+    {
+        return !DEEP || lo ? __ffsll((long long)lo) - 1 : 63 + __ffsll((long long)hi);
+    }
+    __device__ __forceinline__ unsigned group(int l) const
+    {
+        return (unsigned)((!DEEP || l < 16 ? lo : hi) >> (4 * (l & 15))) & 15u;
+    }
+    __device__ __forceinline__ void set_group(int l, unsigned nib)
+    {
+        const int sh = 4 * (l & 15);
+        if (!DEEP || l < 16)
+            lo = (lo & ~(15ull << sh)) | ((unsigned long long)nib << sh);
+        else
+            hi = (hi & ~(15ull << sh)) | ((unsigned long long)nib << sh);
+    }
+    // bits 0 .. p of a word (p = 63: all)
+    static __device__ __forceinline__ unsigned long long upto(int p) { return (2ull << p) - 1ull; }
+    __device__ __forceinline__ void clear_bit(int p)
+    {
+        if (!DEEP || p < 64)
+            lo &= ~(1ull << (p & 63));
+        else
+            hi &= ~(1ull << (p & 63));
+    }
+    __device__ __forceinline__ void clear_upto(int p)
+    {
+        if (!DEEP || p < 64) {
+            lo &= ~upto(p & 63);
+        } else {
+            lo = 0ull;
+            hi &= ~upto(p & 63);
+        }
+    }
+    __device__ __forceinline__ int count_upto(int p) const
+    {
+        if (!DEEP || p < 64)
+            return __popcll(lo & upto(p & 63));
+        return __popcll(lo) + __popcll(hi & upto(p & 63));
+    }
+    __device__ __forceinline__ int count() const { return DEEP ? __popcll(lo) + __popcll(hi) : __popcll(lo); }
+    __device__ __forceinline__ bool has(int p) const
+    {
+        return (((!DEEP || p < 64 ? lo : hi) >> (p & 63)) & 1ull) != 0ull;
+    }
+};
+
 // A parked walk: the ray's position in ObjectIntersector's triangle loop and
-// in DisplacedIntersector's walk, its current t_max and result, its
-// candidate mask and the counters of the triangle in progress.
+// in DisplacedIntersector's walk (the cell last taken and the open groups'
+// bits), its current t_max and result, its candidate mask and the counters
+// of the triangle in progress.
 struct RayState
 {
     double t_max;
-    double ckey; // nearest-first order: the cursor (key, index) of the last triangle taken
+    double ckey; // triangle tree, nearest first: the cursor (key, index) of the last triangle taken
     int cidx;
-    int tri, root, best_tri, flags;
-    int cl, ci, cj, el, ei, ej;
-    int nah, lah;
-    unsigned mask[kMaskWords];
+    int tri, best_tri, flags;
+    int cl, ci, cj;
+    int nah, lah, pad;
+    unsigned long long todo[2], dom[2];
+    unsigned long long mask[4]; // per lane of the ray's four
     // scenes of more than 256 triangles: the buffered candidates, kept
     // across parks so a resumed ray does not walk the tree again
     d32::NearBuf buf;
@@ -366,7 +429,7 @@ struct LeafJob
 };
 // RayState.flags
 constexpr int kFoundInTri = 1; // a hit was taken in the triangle in progress
-constexpr int kResumeHere = 2; // parked before visiting cell `cur` (or at the walk's end): resume without cell_next
+constexpr int kShrunk = 2;     // the leaves of the last job shrank t_max: the cells still open are tested again
 constexpr int kCapped = 4;     // a triangle walk of this ray ran out of its cell-visit cap (DMAP_HIT_CAPPED)
 constexpr int kRerun = 8;      // listed for the filter's schedule (it took a crossing the filter rejects)
 
@@ -393,9 +456,23 @@ __device__ __forceinline__ unsigned long long *round_ctr(unsigned long long *c, 
     return c + 4 * round + k;
 }
 
-// One lane's walk from its parked or fresh state to the next leaf (parked,
-// job written) or to the end of the ray. Every lane of the warp executes one
-// node test per step; lanes that finish take another ray.
+// Four lanes walk one ray (a quad; eight rays per warp), so that the four
+// cells of a sibling group are tested together, one per lane. A lane per ray
+// ran one node test per step with 19.6 of 32 lanes in it, the others being in
+// a pick or between cells; and a ray's tests, one after the other, set the
+// time of small batches and of every launch's tail. Walk rounds and last walk
+// before and after: 64 rays on a quad 212 -> 63 us, 20,011 rays on the sphere
+// of 96 x 512^2 maps 2.80 -> 0.69 ms, 2.80M rays on 96 x 2048^2 34.1 -> 27.2
+// ms. Per quad and step: take
+// the next cell of the open groups (its lowest bit), descend into it by
+// testing its four children, or collect it when it is a leaf.
+//
+// The order, the tests and the leaf jobs are those of the walk that visits
+// one cell at a time: t_max does not change between a group's test and the
+// cells taken from it, except where a job's leaves or a leaf run inline
+// shrink it, and then every group still open is tested again before a cell
+// is taken from it (`stale`).
+//
 // The walk rounds are compiled for DMAP_WALK_MIN_BLOCKS (mask) or
 // DMAP_WALK_TREE_MIN_BLOCKS (tree) CTAs per SM; the last walk (INLINE_LEAF),
 // which runs the few rays left with their leaves inline, for
@@ -404,125 +481,162 @@ __device__ __forceinline__ unsigned long long *round_ctr(unsigned long long *c, 
 #ifndef DMAP_DRAIN_MIN_BLOCKS
 #define DMAP_DRAIN_MIN_BLOCKS 2
 #endif
-template <bool ST, bool INLINE_LEAF, bool TREE, bool NEAR, typename R, typename H, typename Fp>
+template <bool ST, bool INLINE_LEAF, bool TREE, bool NEAR, bool DEEP>
 __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                                                   : (TREE ? DMAP_WALK_TREE_MIN_BLOCKS : DMAP_WALK_MIN_BLOCKS))
     wave_walk(const TriDev32 *__restrict__ tris32, const TriDev *__restrict__ tris64, int n_tri,
-              const AssetDev *__restrict__ assets, const R *__restrict__ rays, int64_t n, dmapk::QueryOpts opt,
-              H *__restrict__ hits, int64_t *__restrict__ stats, RayState *__restrict__ states,
+              const AssetDev *__restrict__ assets, const void *__restrict__ rays, int64_t n, dmapk::QueryOpts opt,
+              void *__restrict__ hits, int64_t *__restrict__ stats, RayState *__restrict__ states,
               const int *__restrict__ q_in, int round, LeafJob *__restrict__ q_leaf, unsigned long long *ctr,
               unsigned *status, int *__restrict__ rerun)
 {
     enum : int { NEED = 0, TOP = 1, WALK = 2, DONE = 3 };
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, sub = lane & 3, lead = lane & 28;
     // the candidates: scenes of up to 256 triangles take a mask of one bit
     // per triangle whose box the ray meets (built by the warp at the ray's
-    // start), larger scenes (TREE) the triangle tree (bvh.cuh), in either
-    // order; the launcher takes the mask only for up to 256 triangles, so its
-    // loops are never compiled into the kernels of larger scenes
-    constexpr bool use_mask = !TREE;
+    // start; triangle t is bit t / 4 of the quad's lane t % 4), larger scenes
+    // (TREE) the triangle tree (bvh.cuh), in either order; the launcher takes
+    // the mask only for up to 256 triangles, so its loops are never compiled
+    // into the kernels of larger scenes
     const d32::BvhView bvh = {opt.bvh_nodes, opt.bvh_tri, opt.bvh_range, opt.bvh_n_nodes};
     // scenes of up to 256 triangles: their object boxes in shared memory
     // (outward FP32 for the box tests, FP64 for the nearest order's keys),
-    // which every candidate test of the CTA reads
+    // which every candidate test of the CTA reads; component c of triangle t
+    // at c * kStaged + t
     constexpr int kStaged = TREE ? 1 : 32 * kMaskWords;
     __shared__ float s_box32[6 * kStaged];
-    __shared__ double s_box64[6 * kStaged];
+    __shared__ double s_box64[(NEAR ? 6 : 1) * kStaged];
     if (!TREE) {
         for (int k = threadIdx.x; k < 6 * n_tri; k += blockDim.x) {
             const int t = k / 6, c = k - 6 * t;
-            s_box32[k] = c < 3 ? tris32[t].box_lo[c] : tris32[t].box_hi[c - 3];
-            s_box64[k] = c < 3 ? tris64[t].box_lo[c] : tris64[t].box_hi[c - 3];
+            s_box32[c * kStaged + t] = c < 3 ? tris32[t].box_lo[c] : tris32[t].box_hi[c - 3];
+            if (NEAR)
+                s_box64[c * kStaged + t] = c < 3 ? tris64[t].box_lo[c] : tris64[t].box_hi[c - 3];
         }
         __syncthreads();
     }
+    auto box32 = [&](int t, float *lo, float *hi) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            lo[c] = s_box32[c * kStaged + t];
+            hi[c] = s_box32[(3 + c) * kStaged + t];
+        }
+    };
     // items of this round: every ray in round 0, else the resume queue
     unsigned long long count = round == 0 ? (unsigned long long)n : *round_ctr(ctr, round - 1, 3);
     if (round == 0 && opt.n_dev && (unsigned long long)*opt.n_dev < count)
         count = *opt.n_dev < 0 ? 0ull : (unsigned long long)*opt.n_dev;
     unsigned long long *fetch = round_ctr(ctr, round, 0);
-    int phase = NEED;
+    // a round of fewer rays than the grid has quads spreads them over all
+    // its warps, so that fewer of them share a warp
+    const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
+    int phase = (unsigned long long)(lane >> 2) * warps < count ? NEED : DONE;
     int ray = 0;
-    double o[3], d[3], t_min = 0.0, t_max = 0.0;
-    float of[3], df[3], invf[3], tmin_f = 0.0f;
-    int tri = 0, best_tri = -1, root = 0, si = 0, sj = 0, nah = 0, lah = 0, flags = 0, guard = 0;
+    double t_max = 0.0;
+    float tmin_f = 0.0f, tmax_f = 0.0f;
+    int tri = 0, best_tri = -1, si = 0, sj = 0, nah = 0, lah = 0, flags = 0, guard = 0;
     double ckey = -INFINITY;
     int cidx = -1;
-    // the triangle tree (TREE): the lane's buffered candidates, refilled
-    // from the ray's cursor for a fresh ray, kept in the ray's state across
-    // parks
+    // the triangle tree (TREE): the buffered candidates, held by the quad's
+    // first lane, refilled from the ray's cursor for a fresh ray, kept in the
+    // ray's state across parks
     d32::NearBuf nbuf;
     nbuf.n = -1;
     nbuf.pos = 0;
     Ray32 r;
-    Cell32 cur = {0, 0, 0}, end = {0, 0, 0};
-    unsigned mask[kMaskWords];
-#pragma unroll
-    for (int w = 0; w < kMaskWords; ++w)
-        mask[w] = 0u;
+    const float *pyr = nullptr;
+    Cell32 cur = {0, 0, 0};
+    CellBits<DEEP> todo = {0ull, 0ull}, dom = {0ull, 0ull}; // cells that passed; cells in the domain, not yet gone past
+    unsigned stale = 0u;                                   // levels whose group must be tested again
+    unsigned long long mask = 0ull;
     int64_t stl[DMAP_ST_N];
-    int nl = 0, li0 = 0, lj0 = 0, li1 = 0, lj1 = 0, li2 = 0, lj2 = 0, li3 = 0, lj3 = 0; // collected leaves
-    int since = 0; // node tests since the first collected leaf
+    int nl = 0, li = 0, lj = 0; // collected leaves, the lane's own
+    int since = 0;              // node tests since the first collected leaf
 
     auto flush_stats = [&]() {
-        if (ST)
+        if (ST && sub == 0)
             for (int q = 0; q < DMAP_ST_N; ++q)
                 stats[DMAP_ST_N * (int64_t)ray + q] += stl[q];
     };
     // Park the ray: its collected leaves become one job, its walk state
-    // waits for the next round (here: resume at `cur` itself, which is the
-    // next cell to visit or the end of the triangle's walk; otherwise `cur`
-    // is the last collected leaf and the walk resumes past it).
-    auto park = [&](bool here) {
+    // waits for the next round.
+    auto park = [&]() {
         RayState &s = states[ray];
-        s.t_max = t_max;
-        s.ckey = ckey;
-        s.cidx = cidx;
-        s.tri = tri;
-        s.root = root;
-        s.best_tri = best_tri;
-        s.flags = here ? (flags | kResumeHere) : (flags & ~kResumeHere);
-        s.cl = cur.level, s.ci = cur.i, s.cj = cur.j;
-        s.el = end.level, s.ei = end.i, s.ej = end.j;
-        s.nah = nah;
-        s.lah = lah;
-#pragma unroll
-        for (int w = 0; w < kMaskWords; ++w)
-            s.mask[w] = mask[w];
-        if (TREE)
-            s.buf = nbuf;
-        unsigned long long slot = atomicAdd(round_ctr(ctr, round, 1), 1ull);
-        LeafJob job;
-        job.ray = ray;
-        job.tri = tri;
-        job.n = nl;
-        job.pad = 0;
-        job.i[0] = li0, job.j[0] = lj0, job.i[1] = li1, job.j[1] = lj1;
-        job.i[2] = li2, job.j[2] = lj2, job.i[3] = li3, job.j[3] = lj3;
-        q_leaf[slot] = job;
+        unsigned long long slot = 0;
+        if (sub == 0) {
+            s.t_max = t_max;
+            s.tri = tri;
+            s.best_tri = best_tri;
+            s.flags = flags;
+            s.cl = cur.level, s.ci = cur.i, s.cj = cur.j;
+            s.todo[0] = todo.lo;
+            s.dom[0] = dom.lo;
+            if (DEEP) {
+                s.todo[1] = todo.hi;
+                s.dom[1] = dom.hi;
+            }
+            if (ST) {
+                s.nah = nah;
+                s.lah = lah;
+            }
+            if (TREE) {
+                s.ckey = ckey;
+                s.cidx = cidx;
+                s.buf = nbuf;
+            }
+            slot = atomicAdd(round_ctr(ctr, round, 1), 1ull);
+        }
+        if (!TREE)
+            s.mask[sub] = mask;
+        slot = __shfl_sync(0xfu << lead, slot, lead);
+        LeafJob &job = q_leaf[slot];
+        if (sub == 0) {
+            job.ray = ray;
+            job.tri = tri;
+            job.n = nl;
+            job.pad = 0;
+        }
+        job.i[sub] = li;
+        job.j[sub] = lj;
         nl = 0;
         since = 0;
         flush_stats();
         phase = NEED;
     };
+    // the ray transform into triangle T's tangent frame, a row per lane
+    auto enter_frame = [&](const TriDev32 &T, const double *o, const double *d, float t_far) {
+        const unsigned quad = 0xfu << lead;
+        float ro, rd, e;
+        tangent_row(T, sub < 3 ? sub : 0, o, d, t_far, ro, rd, e);
+        const float inv = rd != 0.0f ? __frcp_rn(rd) : 0.0f;
+        r.ox = __shfl_sync(quad, ro, lead), r.oy = __shfl_sync(quad, ro, lead + 1), r.oz = __shfl_sync(quad, ro, lead + 2);
+        r.dx = __shfl_sync(quad, rd, lead), r.dy = __shfl_sync(quad, rd, lead + 1), r.dz = __shfl_sync(quad, rd, lead + 2);
+        r.ix = __shfl_sync(quad, inv, lead), r.iy = __shfl_sync(quad, inv, lead + 1), r.iz = __shfl_sync(quad, inv, lead + 2);
+        r.ex = __shfl_sync(quad, e, lead), r.ey = __shfl_sync(quad, e, lead + 1), r.ez = __shfl_sync(quad, e, lead + 2);
+        si = r.dx < 0.0f;
+        sj = r.dy < 0.0f;
+        pyr = T.pyr32;
+    };
 
     for (;;) {
-        // 1. lanes without work take the next items, one atomic per warp
-        unsigned need = __ballot_sync(FULL, phase == NEED);
+        // 1. quads without work take the next items, one atomic per warp
+        const unsigned need = __ballot_sync(FULL, phase == NEED) & 0x11111111u;
         bool fresh = false;
+        float of[3], df[3], invf[3]; // the ray in float, while it is fetched or picks
         if (need) {
-            int leader = __ffs(need) - 1;
+            const int leader = __ffs(need) - 1;
             unsigned long long base = 0;
             if (lane == leader)
                 base = atomicAdd(fetch, (unsigned long long)__popc(need));
             base = __shfl_sync(FULL, base, leader);
             if (phase == NEED) {
-                unsigned long long item = base + (unsigned long long)__popc(need & ((1u << lane) - 1u));
+                unsigned long long item = base + (unsigned long long)__popc(need & ((1u << lead) - 1u));
                 if (item >= count) {
                     phase = DONE;
                 } else {
                     ray = round == 0 ? (int)item : q_in[item];
-                    load_ray(rays, ray, o, d, t_min, t_max);
+                    double o[3], d[3], t_min;
+                    load_ray(rays, opt.ray_dtype, ray, o, d, t_min, t_max);
                     nbuf.n = -1;
 #pragma unroll
                     for (int a = 0; a < 3; ++a) {
@@ -540,37 +654,43 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                         cidx = -1;
                         best_tri = -1;
                         flags = 0;
-                        nah = lah = 0;
+                        mask = 0ull;
+                        tmax_f = __double2float_ru(t_max);
                         fresh = true;
                         phase = TOP;
                     } else {
                         const RayState &s = states[ray];
                         t_max = s.t_max;
-                        ckey = s.ckey;
-                        cidx = s.cidx;
                         tri = s.tri;
-                        root = s.root;
                         best_tri = s.best_tri;
                         flags = s.flags;
-                        nah = s.nah;
-                        lah = s.lah;
-#pragma unroll
-                        for (int w = 0; w < kMaskWords; ++w)
-                            mask[w] = s.mask[w];
-                        if (TREE)
-                            nbuf = s.buf;
-                        // back into the walk just after the leaf (displaced_intersector.cpp:229)
-                        const TriDev32 &T = tris32[tri];
-                        float t1 = __double2float_ru(t_max);
-                        object_box(T, of, df, invf, tmin_f, t1);
-                        tangent_ray(T, o, d, far_bound(fmaxf(t1, tmin_f)), r);
-                        si = r.dx < 0.0f;
-                        sj = r.dy < 0.0f;
                         cur = {s.cl, s.ci, s.cj};
-                        end = {s.el, s.ei, s.ej};
-                        if (!(flags & kResumeHere))
-                            cell_next(cur, si, sj, T.root_level); // past the last leaf (displaced_intersector.cpp:229)
-                        flags &= ~kResumeHere;
+                        todo.lo = s.todo[0];
+                        dom.lo = s.dom[0];
+                        if (DEEP) {
+                            todo.hi = s.todo[1];
+                            dom.hi = s.dom[1];
+                        }
+                        if (ST) {
+                            nah = s.nah;
+                            lah = s.lah;
+                        }
+                        if (TREE) {
+                            ckey = s.ckey;
+                            cidx = s.cidx;
+                            if (sub == 0)
+                                nbuf = s.buf;
+                        } else {
+                            mask = s.mask[sub];
+                        }
+                        // back into the walk just after the leaves (displaced_intersector.cpp:229)
+                        tmax_f = __double2float_ru(t_max);
+                        const TriDev32 &T = tris32[tri];
+                        float t1 = tmax_f;
+                        object_box(T, of, df, invf, tmin_f, t1);
+                        enter_frame(T, o, d, far_bound(fmaxf(t1, tmin_f)));
+                        stale = (flags & kShrunk) ? ~0u : 0u;
+                        flags &= ~kShrunk;
                         guard = 0;
                         nl = 0;
                         phase = WALK;
@@ -578,12 +698,14 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                 }
             }
         }
-        // round 0: the warp finds the fresh rays' candidate triangles together, 32 boxes per ballot
-        if (use_mask) {
-            unsigned todo = __ballot_sync(FULL, fresh);
-            while (todo) {
-                int src = __ffs(todo) - 1;
-                todo &= todo - 1;
+        // round 0: the warp finds the fresh rays' candidate triangles
+        // together, 32 boxes per ballot; byte q of a ballot is the triangles
+        // of lane q
+        if (!TREE) {
+            unsigned left = __ballot_sync(FULL, fresh) & 0x11111111u;
+            while (left) {
+                const int src = __ffs(left) - 1;
+                left &= left - 1;
                 float so[3], sd[3], sv[3];
 #pragma unroll
                 for (int a = 0; a < 3; ++a) {
@@ -591,19 +713,19 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                     sd[a] = __shfl_sync(FULL, df[a], src);
                     sv[a] = __shfl_sync(FULL, invf[a], src);
                 }
-                float s_tmin = __shfl_sync(FULL, tmin_f, src);
-                float s_tmax = __shfl_sync(FULL, __double2float_ru(t_max), src);
+                const float s_tmin = __shfl_sync(FULL, tmin_f, src), s_tmax = __shfl_sync(FULL, tmax_f, src);
 #pragma unroll 1
                 for (int w = 0; w < ((n_tri + 31) >> 5); ++w) {
-                    int t = 32 * w + lane;
-                    float t1 = s_tmax;
-                    bool pass = t < n_tri && box_pass(s_box32 + 6 * t, s_box32 + 6 * t + 3, so, sd, sv, s_tmin, t1);
-                    unsigned bits = __ballot_sync(FULL, pass);
-                    if (lane == src) {
-#pragma unroll
-                        for (int q = 0; q < kMaskWords; ++q)
-                            mask[q] = q == w ? bits : mask[q];
+                    const int t = 32 * w + 4 * (lane & 7) + (lane >> 3);
+                    float t1 = s_tmax, lo[3], hi[3];
+                    bool pass = t < n_tri;
+                    if (pass) {
+                        box32(t, lo, hi);
+                        pass = box_pass(lo, hi, so, sd, sv, s_tmin, t1);
                     }
+                    const unsigned bits = __ballot_sync(FULL, pass);
+                    if (lead == src)
+                        mask |= (unsigned long long)((bits >> (8 * sub)) & 255u) << (8 * w);
                 }
             }
         }
@@ -611,247 +733,316 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
             break;
 
         // 2. the next triangle whose object box the ray meets (intersect_flat's loop)
+        bool test = false, roots = false, again = false; // a group to test: the roots; one tested before
         if (phase == TOP) {
-            float t1 = 0.0f;
-            bool hit_box = false;
-            if (NEAR) {
-                // nearest box entry first: the smallest (key, index) past the
-                // cursor among the candidates the ray still reaches
-                double inv[3];
-                d64::ray_inverse(d, inv);
-                double bk = 0.0;
-                int bt = -1;
-                const float tmf = __double2float_ru(t_max);
-                if (TREE) {
-                    bool err = false;
-                    bt = d32::near_next<true>(nbuf, bvh, tris32, tris64, o, d, inv, t_min, of, df, invf, tmin_f, tmf,
-                                        ckey, cidx, t1, err);
-                    bk = ckey;
-                    if (err)
-                        atomicOr(status, dmapdev::kStatusCapped);
-                } else {
-                    // the best (key, index) past the cursor among the bits
-                    // of the ray's mask (boxes met at the ray's start), each
-                    // box re-tested with the current t_max first; a bit whose
-                    // box no longer passes, or whose key is not past the
-                    // cursor, is cleared for good (t_max only shrinks, the
-                    // cursor only advances), so later picks scan fewer
-                    const int words = (n_tri + 31) >> 5;
-#pragma unroll 1
-                    for (int w = 0; w < words; ++w) {
-                        unsigned bits = mask[0];
+            const unsigned quad = 0xfu << lead;
+            double o[3], d[3], t_min, t_ray;
+            load_ray(rays, opt.ray_dtype, ray, o, d, t_min, t_ray);
+            if (!fresh) {
 #pragma unroll
-                        for (int q = 1; q < kMaskWords; ++q)
-                            bits = w == q ? mask[q] : bits;
-                        unsigned drop = 0u;
-                        while (bits) {
-                            const int b = __ffs(bits) - 1;
-                            bits &= bits - 1;
-                            const int t = 32 * w + b;
-                            float e = tmin_f, tt = tmf;
-                            if (!box_range(s_box32 + 6 * t, s_box32 + 6 * t + 3, of, df, invf, e, tt)) {
-                                drop |= 1u << b;
-                                continue;
-                            }
-                            if (bt >= 0 && (double)e > bk)
-                                continue; // its key (at least e) is past the best
-                            const double key = d64::entry_key(s_box64 + 6 * t, s_box64 + 6 * t + 3, o, d, inv, t_min);
-                            if (!d64::after_cursor(key, t, ckey, cidx)) {
-                                drop |= 1u << b;
-                                continue;
-                            }
-                            if (!d64::before_best(key, t, bk, bt))
-                                continue;
-                            bk = key;
-                            bt = t;
-                            t1 = tt;
-                        }
-                        if (drop) {
-#pragma unroll
-                            for (int q = 0; q < kMaskWords; ++q)
-                                mask[q] = w == q ? (mask[q] & ~drop) : mask[q];
-                        }
-                    }
-                }
-                if (bt >= 0) {
-                    tri = bt;
-                    ckey = bk;
-                    cidx = bt;
-                    hit_box = true;
-                } else {
-                    tri = n_tri;
-                }
-            } else if (TREE) {
-                // index order: the smallest index from tri on whose box the
-                // ray still meets
-                bool err = false;
-                double ck = tri - 1;
-                int ci = tri - 1;
-                const int t = d32::near_next<false>(nbuf, bvh, tris32, tris64, o, d, nullptr, t_min, of, df, invf,
-                                                    tmin_f, __double2float_ru(t_max), ck, ci, t1, err);
-                if (err)
-                    atomicOr(status, dmapdev::kStatusCapped);
-                if (t >= 0) {
-                    tri = t;
-                    hit_box = true;
-                } else {
-                    tri = n_tri;
-                }
-            } else {
-                while (tri < n_tri) {
-                    int w = tri >> 5;
-                    unsigned bits = mask[0];
-#pragma unroll
-                    for (int q = 1; q < kMaskWords; ++q)
-                        bits = w == q ? mask[q] : bits;
-                    bits &= ~0u << (tri & 31);
-                    if (!bits) {
-                        tri = (w + 1) << 5;
-                        continue;
-                    }
-                    tri = (w << 5) + __ffs(bits) - 1;
-                    t1 = __double2float_ru(t_max); // the candidate again, with the current t_max
-                    if (tri < n_tri && box_pass(s_box32 + 6 * tri, s_box32 + 6 * tri + 3, of, df, invf, tmin_f, t1)) {
-                        hit_box = true;
-                        break;
-                    }
-                    ++tri;
+                for (int a = 0; a < 3; ++a) {
+                    of[a] = (float)o[a];
+                    df[a] = (float)d[a];
+                    invf[a] = df[a] != 0.0f ? __frcp_rn(df[a]) : 0.0f;
                 }
             }
-            if (!hit_box) {
-                if (best_tri < 0) {
-                    d64::hit64 none;
-                    store_hit<H, Fp>(hits, ray, false, none, -1, (flags & kCapped) ? DMAP_HIT_CAPPED : 0);
-                } else if (flags & kCapped) {
-                    hits[ray].flags |= DMAP_HIT_CAPPED; // the stored hit is final: this lane owns the ray
+            float t1 = 0.0f;
+            int bt = -1;
+            double inv[3];
+            if (NEAR) {
+                // 1 / d in double, an axis per lane
+                const double da = sub == 0 ? d[0] : sub == 1 ? d[1] : d[2];
+                const double ia = da != 0.0 ? 1.0 / da : 0.0;
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+                    inv[a] = __shfl_sync(quad, ia, lead + a);
+            }
+            if (TREE) {
+                if (sub == 0) {
+                    bool err = false;
+                    if (NEAR) {
+                        bt = d32::near_next<true>(nbuf, bvh, tris32, tris64, o, d, inv, t_min, of, df, invf, tmin_f,
+                                                  tmax_f, ckey, cidx, t1, err);
+                    } else {
+                        // index order: the smallest index from tri on whose
+                        // box the ray still meets
+                        double ck = tri - 1;
+                        int ci = tri - 1;
+                        bt = d32::near_next<false>(nbuf, bvh, tris32, tris64, o, d, nullptr, t_min, of, df, invf,
+                                                   tmin_f, tmax_f, ck, ci, t1, err);
+                    }
+                    if (err)
+                        atomicOr(status, dmapdev::kStatusCapped);
+                }
+                bt = __shfl_sync(quad, bt, lead);
+                t1 = __shfl_sync(quad, t1, lead);
+                ckey = __shfl_sync(quad, ckey, lead);
+                cidx = __shfl_sync(quad, cidx, lead);
+            } else {
+                // the best of each lane's candidates (nearest order: the
+                // smallest (key, index); index order: the smallest index),
+                // then of the quad's; each box is re-tested with the current
+                // t_max first, and a bit whose box no longer passes is
+                // cleared for good (t_max only shrinks). The taken triangle's
+                // bit is cleared too, so every bit left is past it.
+                double bk = 0.0;
+                unsigned long long m = mask;
+                while (m) {
+                    const int b = __ffsll((long long)m) - 1;
+                    m &= m - 1ull;
+                    const int t = 4 * b + sub;
+                    float e = tmin_f, tt = tmax_f, lo[3], hi[3];
+                    box32(t, lo, hi);
+                    if (!box_range(lo, hi, of, df, invf, e, tt)) {
+                        mask &= ~(1ull << b);
+                        continue;
+                    }
+                    if (!NEAR) {
+                        bt = t;
+                        t1 = tt;
+                        break;
+                    }
+                    if (bt >= 0 && (double)e > bk)
+                        continue; // its key (at least e) is past the best
+                    double dlo[3], dhi[3];
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        dlo[c] = s_box64[c * kStaged + t];
+                        dhi[c] = s_box64[(3 + c) * kStaged + t];
+                    }
+                    const double key = d64::entry_key(dlo, dhi, o, d, inv, t_min);
+                    if (!d64::before_best(key, t, bk, bt))
+                        continue;
+                    bk = key;
+                    bt = t;
+                    t1 = tt;
+                }
+                __syncwarp(quad);
+#pragma unroll
+                for (int x = 1; x < 4; x <<= 1) {
+                    const int ot = __shfl_xor_sync(quad, bt, x);
+                    const float o1 = __shfl_xor_sync(quad, t1, x);
+                    const double ok = NEAR ? __shfl_xor_sync(quad, bk, x) : (double)ot;
+                    if (ot >= 0 && (NEAR ? d64::before_best(ok, ot, bk, bt) : (bt < 0 || ot < bt))) {
+                        bk = ok;
+                        bt = ot;
+                        t1 = o1;
+                    }
+                }
+                if (bt >= 0 && (bt & 3) == sub)
+                    mask &= ~(1ull << (bt >> 2));
+            }
+            if (bt < 0) {
+                if (sub == 0) {
+                    if (best_tri < 0) {
+                        d64::hit64 none;
+                        store_hit(hits, opt.hit_dtype, ray, false, none, -1, (flags & kCapped) ? DMAP_HIT_CAPPED : 0);
+                    } else if (flags & kCapped) {
+                        // the stored hit is final: this quad owns the ray
+                        if (opt.hit_dtype == 2)
+                            static_cast<dmapdev::Hit64 *>(hits)[ray].flags |= DMAP_HIT_CAPPED;
+                        else
+                            static_cast<dmapdev::Hit32 *>(hits)[ray].flags |= DMAP_HIT_CAPPED;
+                    }
                 }
                 flush_stats();
                 phase = NEED;
             } else {
-                const TriDev32 &T = tris32[tri];
-                tangent_ray(T, o, d, far_bound(t1), r);
-                si = r.dx < 0.0f;
-                sj = r.dy < 0.0f;
-                root = 0;
-                cur = {T.root_level, T.roots_i[0], T.roots_j[0]};
-                end = cur;
-                cell_next(end, si, sj, T.root_level);
+                tri = bt;
+                enter_frame(tris32[tri], o, d, far_bound(t1));
+                todo = {0ull, 0ull};
+                dom = {0ull, 0ull};
+                stale = 0u;
                 guard = 0;
                 flags &= ~kFoundInTri;
                 nah = lah = 0;
                 if (ST)
                     ++stl[DMAP_ST_TRI];
                 phase = WALK;
-            }
-        }
-
-        // 3a. advance to the next cell inside the domain (cheap, divergent)
-        bool cand = false;
-        if (phase == WALK) {
-            const TriDev32 &T = tris32[tri];
-            const int log2n = __ffs(assets[T.asset].n_leaf) - 1;
-            for (;;) {
-                if (cur.level == end.level && cur.i == end.i && cur.j == end.j) {
-                    if (root + 1 < T.n_roots) {
-                        ++root;
-                        cur = {T.root_level, T.roots_i[root], T.roots_j[root]};
-                        end = cur;
-                        cell_next(end, si, sj, T.root_level);
-                        continue;
-                    }
-                    if (!INLINE_LEAF && nl > 0) {
-                        // the collected leaves decide this triangle's t_max before the next one
-                        park(true);
-                        break;
-                    }
-                    if (ST && (flags & kFoundInTri)) {
-                        stl[DMAP_ST_NAH] += nah;
-                        stl[DMAP_ST_LAH] += lah;
-                    }
-                    ++tri;
-                    phase = TOP;
-                    break;
-                }
-                if (++guard > opt.guard_cap) { // a finite tree: the cap guards corrupt records
-                    atomicOr(status, dmapdev::kStatusCapped);
-                    flags |= kCapped;
-                    ++tri;
-                    phase = TOP;
-                    break;
-                }
-                float w = pow2f(cur.level - log2n);
-                if (!square_meets_domain(T, ((float)cur.i + 0.5f) * w, ((float)cur.j + 0.5f) * w, 0.5f * w)) {
-                    cell_next(cur, si, sj, T.root_level);
-                    continue;
-                }
-                cand = true;
-                break;
+                test = roots = true;
             }
         }
         __syncwarp();
 
-        // 3b. one node test for every lane with a candidate, all together
-        if (cand) {
-            const TriDev32 &T = tris32[tri];
-            if (ST) {
-                ++stl[DMAP_ST_NODE];
-                ++nah;
+        // 3a. the next cell of the open groups: a leaf is collected, another
+        // cell's children are the group to test
+        int tl = 0, pi = 0, pj = 0; // the group: its level, its parent cell
+        unsigned cells = 15u;
+        bool leaf = false;
+        if (phase == WALK) {
+            const int root_level = tris32[tri].root_level;
+            if (test) {
+                tl = root_level;
+                cells = (1u << tris32[tri].n_roots) - 1u;
+                if (DEEP && tl > 31) { // beyond the bits of the open groups
+                    atomicOr(status, dmapdev::kStatusCapped);
+                    flags |= kCapped;
+                    ++tri;
+                    phase = TOP;
+                    test = false;
+                }
             }
-            if (!node_test32(T, assets[T.asset], r, cur.level, cur.i, cur.j, tmin_f, __double2float_ru(t_max),
-                             opt.bound, opt.slab_max_level)) {
-                cell_next(cur, si, sj, T.root_level);
-            } else if (cur.level > 0) {
-                --cur.level;
-                cur.i = 2 * cur.i + si;
-                cur.j = 2 * cur.j + sj;
-            } else {
+            while (!test && phase == WALK) {
+                if (!todo.any()) {
+                    // the end of the triangle's walk
+                    if (ST) {
+                        const int left = dom.count();
+                        stl[DMAP_ST_NODE] += left;
+                        nah += left;
+                    }
+                    dom = {0ull, 0ull};
+                    if (!INLINE_LEAF && nl > 0) {
+                        // the collected leaves decide this triangle's t_max before the next one
+                        park();
+                    } else {
+                        if (ST && (flags & kFoundInTri)) {
+                            stl[DMAP_ST_NAH] += nah;
+                            stl[DMAP_ST_LAH] += lah;
+                        }
+                        ++tri;
+                        phase = TOP;
+                    }
+                    break;
+                }
+                const int p = todo.first(), l = p >> 2, k = p & 3, sh = l + 1 - cur.level;
+                const bool at_root = l == root_level;
+                pi = at_root ? 0 : cur.i >> sh;
+                pj = at_root ? 0 : cur.j >> sh;
+                if ((stale >> l) & 1u) {
+                    // its group was tested with a t_max that has shrunk since
+                    tl = l;
+                    cells = todo.group(l);
+                    roots = at_root;
+                    test = again = true;
+                    break;
+                }
+                // the tests the one-cell walk makes from the last cell taken
+                // to this one: the cells in the domain between them that
+                // failed, and this one (unless it was counted before a park)
+                const int n_in = dom.count_upto(p);
+                if (!INLINE_LEAF && nl > 0) {
+                    const int before = n_in - (dom.has(p) ? 1 : 0);
+                    if (since + before > DMAP_STALE_CAP) {
+                        // the ray holds collected leaves and walked on for
+                        // DMAP_STALE_CAP tests with the t_max it had before
+                        // them: park, so that they can shrink it
+                        if (ST) {
+                            for (int q = DMAP_STALE_CAP + 1 - since; q > 0; --q) {
+                                dom.clear_bit(dom.first());
+                                ++stl[DMAP_ST_NODE];
+                                ++nah;
+                            }
+                        }
+                        park();
+                        break;
+                    }
+                    since += n_in;
+                }
+                if (ST) {
+                    stl[DMAP_ST_NODE] += n_in;
+                    nah += n_in;
+                }
+                dom.clear_upto(p);
+                if (l > 0 && nl > 0 && since > DMAP_STALE_CAP) {
+                    park(); // the cell is taken (and its group tested) again after the resume
+                    break;
+                }
+                todo.clear_bit(p);
+                const TriDev32 &T = tris32[tri];
+                cur.level = l;
+                cur.i = at_root ? T.roots_i[k] : 2 * pi + ((k >> 1) ^ si);
+                cur.j = at_root ? T.roots_j[k] : 2 * pj + ((k & 1) ^ sj);
+                if (l > 0) {
+                    tl = l - 1;
+                    pi = cur.i;
+                    pj = cur.j;
+                    test = true;
+                    break;
+                }
                 if (ST) {
                     ++stl[DMAP_ST_LEAF];
                     ++lah;
                 }
                 if (INLINE_LEAF) {
-                    // the last round: the few remaining rays finish here
-                    d64::hit64 lh;
-                    int lf = 0;
-                    if (leaf_cell(T, tris64[tri], assets[T.asset], o, d, t_min, t_max, cur.i, cur.j, lh, lf,
-                                  ST ? stl : nullptr, opt) &&
-                        lh.t < t_max) {
-                        t_max = lh.t;
-                        best_tri = tri;
-                        flags |= kFoundInTri;
-                        nah = lah = 0;
-                        store_hit<H, Fp>(hits, ray, true, lh, tri, lf | ((flags & kCapped) ? DMAP_HIT_CAPPED : 0));
-                        check_crossing(opt, tris64[tri], tri, lh, ray, flags, ctr, rerun);
-                        if (opt.mode == 1) {
-                            flush_stats();
-                            phase = NEED;
-                        }
-                    }
-                    if (phase == WALK)
-                        cell_next(cur, si, sj, T.root_level);
-                } else {
-                    // collect the leaf; park once kCollect are held
-                    li0 = nl == 0 ? cur.i : li0;
-                    lj0 = nl == 0 ? cur.j : lj0;
-                    li1 = nl == 1 ? cur.i : li1;
-                    lj1 = nl == 1 ? cur.j : lj1;
-                    li2 = nl == 2 ? cur.i : li2;
-                    lj2 = nl == 2 ? cur.j : lj2;
-                    li3 = nl == 3 ? cur.i : li3;
-                    lj3 = nl == 3 ? cur.j : lj3;
-                    if (++nl == DMAP_COLLECT)
-                        park(false);
-                    else
-                        cell_next(cur, si, sj, T.root_level);
+                    leaf = true;
+                    break;
+                }
+                // collect the leaf; park once DMAP_COLLECT are held
+                if (sub == nl) {
+                    li = cur.i;
+                    lj = cur.j;
+                }
+                if (nl == 0)
+                    since = 1;
+                if (++nl == DMAP_COLLECT || since > DMAP_STALE_CAP)
+                    park();
+            }
+        }
+        __syncwarp();
+
+        if (INLINE_LEAF) {
+            // the last round: the few remaining rays finish here
+            int got = 0;
+            if (leaf && sub == 0) {
+                double o[3], d[3], t_min, t_ray;
+                load_ray(rays, opt.ray_dtype, ray, o, d, t_min, t_ray);
+                d64::hit64 lh;
+                int lf = 0;
+                if (leaf_cell(tris32[tri], tris64[tri], assets[tris32[tri].asset], o, d, t_min, t_max, cur.i, cur.j, lh,
+                              lf, ST ? stl : nullptr, opt) &&
+                    lh.t < t_max) {
+                    t_max = lh.t;
+                    got = 1;
+                    store_hit(hits, opt.hit_dtype, ray, true, lh, tri, lf | ((flags & kCapped) ? DMAP_HIT_CAPPED : 0));
+                    check_crossing(opt, tris64[tri], tri, lh, ray, flags, ctr, rerun);
+                }
+            }
+            __syncwarp();
+            got = __shfl_sync(FULL, got, lead);
+            t_max = __shfl_sync(FULL, t_max, lead);
+            flags = __shfl_sync(FULL, flags, lead);
+            if (leaf && got) {
+                tmax_f = __double2float_ru(t_max);
+                best_tri = tri;
+                flags |= kFoundInTri;
+                nah = lah = 0;
+                stale = ~0u;
+                if (opt.mode == 1) {
+                    flush_stats();
+                    phase = NEED;
                 }
             }
         }
-        // a ray holding collected leaves walks on with the t_max it had
-        // before them; after DMAP_STALE_CAP such node tests it parks (at the
-        // next cell to visit) so that the leaves can shrink t_max first
-        if (!INLINE_LEAF && phase == WALK && nl > 0 && ++since > DMAP_STALE_CAP)
-            park(true);
-        __syncwarp();
+
+        // 3b. the group's cells, one per lane, all quads together
+        bool in = false, pass = false;
+        if (test && ((cells >> sub) & 1u)) {
+            const TriDev32 &T = tris32[tri];
+            const Walk32 W = load_walk(T);
+            const int ci = roots ? T.roots_i[sub] : 2 * pi + ((sub >> 1) ^ si);
+            const int cj = roots ? T.roots_j[sub] : 2 * pj + ((sub & 1) ^ sj);
+            const float w = pow2f(tl - W.log2n);
+            in = square_meets_domain(W, ((float)ci + 0.5f) * w, ((float)cj + 0.5f) * w, 0.5f * w);
+            if (in)
+                pass = node_test32(W, pyr, r, tl, ci, cj, tmin_f, tmax_f, opt.bound, opt.slab_max_level);
+        }
+        const unsigned b_in = __ballot_sync(FULL, in), b_pass = __ballot_sync(FULL, pass);
+        if (test) {
+            todo.set_group(tl, (b_pass >> lead) & 15u);
+            stale &= ~(1u << tl);
+            if (!again) {
+                dom.set_group(tl, (b_in >> lead) & 15u);
+                if (roots)
+                    cur = {tl + 1, 0, 0};
+                guard += __popc(cells);
+                if (guard > opt.guard_cap) { // a finite tree: the cap guards corrupt records
+                    atomicOr(status, dmapdev::kStatusCapped);
+                    flags |= kCapped;
+                    todo = {0ull, 0ull};
+                    dom = {0ull, 0ull};
+                }
+            }
+        }
     }
 }
 
@@ -1071,7 +1262,7 @@ __global__ void __launch_bounds__(128, DMAP_LEAF_MIN_BLOCKS)
                 RayState &s = states[ray];
                 s.t_max = h.t;
                 s.best_tri = tri;
-                s.flags |= kFoundInTri;
+                s.flags |= kFoundInTri | kShrunk;
                 s.nah = s.lah = 0;
                 if (tris64[tri].inst)
                     dmapdev::world_normal(opt.inst_xf + dmapdev::kInstDoubles * (tris64[tri].inst - 1), h.ng);
@@ -1236,7 +1427,7 @@ __global__ void __launch_bounds__(128, DMAP_LEAF32_MIN_BLOCKS)
                 RayState &s = states[ray];
                 s.t_max = h.t;
                 s.best_tri = tri;
-                s.flags |= kFoundInTri;
+                s.flags |= kFoundInTri | kShrunk;
                 s.nah = s.lah = 0;
                 if (tris64[tri].inst)
                     dmapdev::world_normal(opt.inst_xf + dmapdev::kInstDoubles * (tris64[tri].inst - 1), h.ng);

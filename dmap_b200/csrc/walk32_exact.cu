@@ -33,27 +33,26 @@ cudaError_t simple_rerun(const Args &a, cudaStream_t stream)
     return cudaGetLastError();
 }
 
-template <typename R, typename H, typename Fp>
 cudaError_t walk_drain(const Args &a, const int *q_in, int round, cudaStream_t stream)
 {
     const bool nearest = a.opt.order == 1, tree = a.n_tri > 32 * kMaskWords;
-    const R *rr = static_cast<const R *>(a.rays);
-    H *hh = static_cast<H *>(a.hits);
     RayState *states = static_cast<RayState *>(a.states);
     LeafJob *leaves = static_cast<LeafJob *>(a.leaves);
-#define DMAP_DRAIN(ST_, TR_, NR_)                                                                                   \
-    wave_walk<ST_, true, TR_, NR_, R, H, Fp><<<a.grid, 128, 0, stream>>>(a.t32, a.t64, a.n_tri, a.assets, rr, a.n,  \
-                                                                         a.opt, hh, ST_ ? a.stats : nullptr,       \
-                                                                         states, q_in, round, leaves, a.counters,  \
-                                                                         a.status, a.rerun)
+#define DMAP_DRAIN(ST_, TR_, NR_, DP_)                                                                              \
+    wave_walk<ST_, true, TR_, NR_, DP_><<<a.grid, 128, 0, stream>>>(                                     \
+        a.t32, a.t64, a.n_tri, a.assets, a.rays, a.n, a.opt, a.hits, ST_ ? a.stats : nullptr, states, q_in, round, leaves,  \
+        a.counters, a.status, a.rerun)
+#define DMAP_DRAIN_DEEP(ST_, TR_, NR_)                                                                              \
+    (ST_ || a.opt.deep ? DMAP_DRAIN(ST_, TR_, NR_, true) : DMAP_DRAIN(false, TR_, NR_, false))
 #define DMAP_DRAIN_MODE(ST_)                                                                                        \
-    (tree ? (nearest ? DMAP_DRAIN(ST_, true, true) : DMAP_DRAIN(ST_, true, false))                                  \
-          : (nearest ? DMAP_DRAIN(ST_, false, true) : DMAP_DRAIN(ST_, false, false)))
+    (tree ? (nearest ? DMAP_DRAIN_DEEP(ST_, true, true) : DMAP_DRAIN_DEEP(ST_, true, false))                        \
+          : (nearest ? DMAP_DRAIN_DEEP(ST_, false, true) : DMAP_DRAIN_DEEP(ST_, false, false)))
     if (a.stats)
         DMAP_DRAIN_MODE(true);
     else
         DMAP_DRAIN_MODE(false);
 #undef DMAP_DRAIN_MODE
+#undef DMAP_DRAIN_DEEP
 #undef DMAP_DRAIN
     return cudaGetLastError();
 }
@@ -104,7 +103,6 @@ cudaError_t leaf32(const Args &a, int round, int *q_out, cudaStream_t stream)
 #define DMAP_W32_EXACT(R, H, Fp)                                                                                    \
     template cudaError_t simple<R, H, Fp>(const Args &, cudaStream_t);                                              \
     template cudaError_t simple_rerun<R, H, Fp>(const Args &, cudaStream_t);                                        \
-    template cudaError_t walk_drain<R, H, Fp>(const Args &, const int *, int, cudaStream_t);                        \
     template cudaError_t leaf64<R, H, Fp>(const Args &, int, int *, cudaStream_t);                                  \
     template cudaError_t leaf32<R, H, Fp>(const Args &, int, int *, cudaStream_t);
 DMAP_W32_EXACT(float, dmapdev::Hit32, float)

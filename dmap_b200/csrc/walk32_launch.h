@@ -38,7 +38,6 @@ cudaError_t simple(const Args &a, cudaStream_t stream);
 // the filter's schedule over the rays a filtered wavefront query listed
 template <typename R, typename H, typename Fp>
 cudaError_t simple_rerun(const Args &a, cudaStream_t stream);
-template <typename R, typename H, typename Fp>
 cudaError_t walk_drain(const Args &a, const int *q_in, int round, cudaStream_t stream);
 template <typename R>
 cudaError_t filter(const Args &a, int round, cudaStream_t stream);
@@ -48,7 +47,6 @@ template <typename R, typename H, typename Fp>
 cudaError_t leaf32(const Args &a, int round, int *q_out, cudaStream_t stream);
 
 // walk32.cu
-template <typename R, typename H, typename Fp>
 cudaError_t walk_round(const Args &a, const int *q_in, int round, cudaStream_t stream);
 
 } // namespace w32

@@ -1,0 +1,78 @@
+"""The wavefront walk's groups of four lanes per ray, where they can go
+wrong: batches that fill no warp, one warp and a ragged number of them;
+triangle counts around the 32 boxes of a ballot and the last one of the
+candidate mask; charts whose root level is past the 64 bits of open groups
+(the wider bits), mirrored and off the cell lattice. Every record equals the
+oracle's bit for bit with the FP64 leaf, in both orders."""
+import numpy as np
+import pytest
+
+import dmap_b200 as dm
+import py_oracle
+import helpers
+from dmap_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    return dm.Context(0)
+
+
+def _equal(cpu, dev, rays, order, rounds):
+    ho, _ = cpu.intersect(rays, order=order)
+    hd = dev.intersect(rays, dm.TraversalOptions(order=order, rounds=rounds, leaf_precision="f64"), np.float64)
+    hit = ho[:, 10] >= 0
+    assert np.array_equal(hd["tri"], np.where(hit, ho[:, 10], -1).astype(np.int32))
+    assert np.array_equal(hd["t"][hit], ho[hit, 0]) and np.array_equal(hd["st"][hit], ho[hit, 1:3])
+    assert np.array_equal(hd["ng"][hit], ho[hit, 5:8])
+    assert np.array_equal(hd["i"][hit], ho[hit, 8].astype(np.int32))
+    return int(hit.sum())
+
+
+@pytest.mark.parametrize("order", ["nearest", "index"])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 33, 1025])
+def test_batch_sizes(ctx, oracle, n, order):
+    sc = helpers.small_sphere(16)
+    cpu, dev = py_oracle.CpuScene(oracle, sc), dm.Scene.from_synthetic(ctx, sc)
+    rays = helpers.near_surface_rays(cpu, n, seed=n)
+    for rounds in (0, 1, 2):
+        _equal(cpu, dev, rays, order, rounds)
+
+
+@pytest.mark.parametrize("order", ["nearest", "index"])
+@pytest.mark.parametrize("tris", [2, 30, 32, 34, 254, 256])
+def test_candidate_mask_edges(ctx, oracle, tris, order):
+    sc = scenes.cube_sphere_scene(4, 5, patches=list(range(tris // 2)))
+    cpu, dev = py_oracle.CpuScene(oracle, sc), dm.Scene.from_synthetic(ctx, sc)
+    assert dev.n_tri == tris
+    rays = np.concatenate([helpers.near_surface_rays(cpu, 400, seed=tris), helpers.aimed_rays(cpu, 200)[0]])
+    assert _equal(cpu, dev, rays, order, 2) > 100
+
+
+@pytest.mark.parametrize("rounds", [0, 2])
+@pytest.mark.parametrize("tiles", [1500, 3000, 12000])
+def test_deep_charts(ctx, oracle, tiles, rounds):
+    """A repeated 32 x 32 map over up to 12,000 tiles a side: root levels 15 (64 bits), 16 and 18."""
+    h = scenes.sine_noise_heights(32, 5, 0.3)
+    asset = scenes.Asset(scenes.close_tile(h, repeat=True).astype(np.float32), repeat=True)
+    z = np.array([0.0, 0.0, 1.0])
+    s = float(tiles)
+    tri = np.concatenate([[0, 0, 0], [s, 0.1, 0], [0.2, s, 0], z, z, z, [0.3, 0.4], [s + 0.3, 0.7], [0.9, s + 0.4]])
+    flip = np.concatenate([[0, 0, 3.0], [s, 0.1, 3.0], [0.2, s, 3.0], z, z, z, [0.3, 0.4], [0.9, s + 0.4],
+                           [s + 0.3, 0.7]])
+    sc = scenes.Scene([asset], np.stack([tri, flip]), np.zeros(2, np.int32), name="deep", extent=s)
+    cpu, dev = py_oracle.CpuScene(oracle, sc), dm.Scene.from_synthetic(ctx, sc)
+    rng = np.random.default_rng(tiles)
+    n = 300
+    p = rng.random((n, 2)) * 0.45 * s
+    rays = np.zeros((n, 8), np.float32)
+    rays[:, 0:2], rays[:, 2] = p, rng.choice([-1.0, 1.5, 4.5], n)
+    d = rng.normal(size=(n, 3))
+    d[:, 2] = np.sign(1.5 - rays[:, 2] + 1e-3) * (0.3 + np.abs(d[:, 2]))
+    rays[:, 3:6], rays[:, 7] = d, np.inf
+    levels = {1500: 15, 3000: 16, 12000: 18}
+    assert dev.triangle_info(0)[0] == levels[tiles]
+    for order in ("nearest", "index"):
+        assert _equal(cpu, dev, rays, order, rounds) > 100
