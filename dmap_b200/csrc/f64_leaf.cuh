@@ -79,7 +79,39 @@ __device__ inline bool newton_from(const TriDev &T, const AssetDev &g, v3 o, v3 
     return false;
 }
 
-struct leafbound { v2 lo; double w, h00, h10, h01, h11; af3 N_hat; v3 o, dn, d1, d2; double d_len; };
+// The hit record at a root (t, st): barycentrics and the reference's normal,
+// Su x Sv there, as newton_from evaluates them (:356-364).
+__device__ inline void root_record(const TriDev &T, const AssetDev &g, double t, v2 st, int64_t i, int64_t j, hit64 &hit)
+{
+    nframe f = normal_frame_at(T, st.x, st.y);
+    double h;
+    v2 gh;
+    grid_h_grad(g, st.x, st.y, h, gh);
+    v3 Su = add3(add3(L3(T.e1), mul3(gh.x, f.N)), mul3(h, f.Nu));
+    v3 Sv = add3(add3(L3(T.e2), mul3(gh.y, f.N)), mul3(h, f.Nv));
+    hit.t = t;
+    hit.st = st;
+    hit.bary = tri_bary(T, st.x, st.y);
+    hit.ng = normalized3(cross3(Su, Sv));
+    hit.i = i;
+    hit.j = j;
+}
+
+// What a leaf's setup computes (208 bytes, thirteen 16-byte words), and with
+// the texel and the ray's origin, which follow from the cell and the ray.
+struct alignas(16) leafrec { double h00, h10, h01, h11; af3 N_hat; v3 dn, d1, d2; double d_len; };
+static_assert(sizeof(leafrec) == 208, "leaf record");
+struct leafbound : leafrec
+{
+    v2 lo;
+    double w;
+    v3 o;
+    __device__ __forceinline__ void place(const AssetDev &g, int64_t i, int64_t j)
+    {
+        w = cell_width(g, 0);
+        lo = {i * w, j * w};
+    }
+};
 
 __device__ __forceinline__ af restricted(af f, double a, double b, double rho) // :72-76
 {
@@ -115,18 +147,11 @@ __device__ inline bool sub_square_bound(const TriDev &T, const leafbound &L, dou
 
 struct leafent { double a, b, t_lo; int depth; };
 
-// intersect_newton + search_leaf (:239-264, :292-323) with an explicit
-// stack: a popped entry is a call of search_leaf at its depth; siblings are
-// pushed in reverse sorted order so the nearest comes off first, and the
-// t_lo >= t_max test at the pop equals the sorted loop's break, since t_max
-// only shrinks.
-__device__ inline bool intersect_newton(const TriDev &T, const AssetDev &g, v3 o, v3 d, double t_min, double t_max,
-                                 int64_t i, int64_t j, hit64 &hit, int64_t *st)
+// intersect_newton's setup (:239-264): the texel's corners, its normal form
+// and the ray's plane basis.
+__device__ inline void leaf_setup(const TriDev &T, const AssetDev &g, v3 o, v3 d, int64_t i, int64_t j, leafbound &L)
 {
-    constexpr int kDepth = 5; // subdivision_depth
-    leafbound L;
-    L.w = cell_width(g, 0);
-    L.lo = {i * L.w, j * L.w};
+    L.place(g, i, j);
     L.h00 = grid_h(g, L.lo.x, L.lo.y);
     L.h10 = grid_h(g, L.lo.x + L.w, L.lo.y);
     L.h01 = grid_h(g, L.lo.x, L.lo.y + L.w);
@@ -140,6 +165,19 @@ __device__ inline bool intersect_newton(const TriDev &T, const AssetDev &g, v3 o
     L.d_len = norm3(d);
     L.dn = div3(d, L.d_len);
     plane_basis(L.dn, L.d1, L.d2);
+}
+
+// intersect_newton + search_leaf (:239-264, :292-323) with an explicit
+// stack: a popped entry is a call of search_leaf at its depth; siblings are
+// pushed in reverse sorted order so the nearest comes off first, and the
+// t_lo >= t_max test at the pop equals the sorted loop's break, since t_max
+// only shrinks.
+__device__ inline bool intersect_newton(const TriDev &T, const AssetDev &g, v3 o, v3 d, double t_min, double t_max,
+                                 int64_t i, int64_t j, hit64 &hit, int64_t *st)
+{
+    constexpr int kDepth = 5; // subdivision_depth
+    leafbound L;
+    leaf_setup(T, g, o, d, i, j, L);
 
     bool found = false;
     int64_t subs = 0, iters = 0;

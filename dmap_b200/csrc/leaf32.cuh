@@ -43,9 +43,10 @@ using namespace d64;
 
 constexpr float kG2 = 2.0f * d32::G; // margin factor of the bound's terms
 
-struct Leaf32
+// What the setup computes (192 bytes: kept as twelve 16-byte words between
+// the kernel that sets leaves up and the one that searches them).
+struct alignas(16) Rec32
 {
-    double lo_s, lo_t, w; // the texel in chart coordinates
     double Q3, inv_dlen;  // dn . (X0 - o) and 1 / |d|, in double
     float q0, q1;         // d1 . (X0 - o), d2 . (X0 - o)
     // along d1, d2, dn (index k): P(a, b) - P(c0) = alpha pe1 + beta pe2
@@ -58,15 +59,24 @@ struct Leaf32
     float hmid, d00, ha, hb, tw; // h(a, b) = hmid + d00 + ha a + hb b + tw a b
     float tol2;           // Newton acceptance: residual^2 below this
 };
+static_assert(sizeof(Rec32) == 192, "leaf record");
+
+struct Leaf32 : Rec32
+{
+    double lo_s, lo_t, w; // the texel in chart coordinates
+    __device__ __forceinline__ void place(const AssetDev &g, int64_t i, int64_t j)
+    {
+        w = cell_width(g, 0);
+        lo_s = i * w;
+        lo_t = j * w;
+    }
+};
 
 // intersect_newton's setup (:239-264) and the leaf's FP32 terms.
 __device__ inline void leaf_setup32(const TriDev &T, const AssetDev &g, v3 o, v3 d, int64_t i, int64_t j, Leaf32 &L)
 {
-    double w = cell_width(g, 0);
-    double los = i * w, lot = j * w;
-    L.lo_s = los;
-    L.lo_t = lot;
-    L.w = w;
+    L.place(g, i, j);
+    const double w = L.w, los = L.lo_s, lot = L.lo_t;
     double h00 = grid_h(g, los, lot), h10 = grid_h(g, los + w, lot);
     double h01 = grid_h(g, los, lot + w), h11 = grid_h(g, los + w, lot + w);
     double hm = 0.25 * ((h00 + h10) + (h01 + h11));
@@ -250,23 +260,25 @@ __device__ inline bool newton32(const TriDev &T, const Leaf32 &L, float a, float
     return false;
 }
 
-// An FP32 root as a hit (newton_from's acceptance tests, :350-364), with the
-// FP64 polish when the Jacobian is ill-conditioned. The texel (lo_s, lo_t,
-// w) and the ray's Q3 and 1/|d| come from the leaf's setup. flags gets
+// An FP32 root judged (newton_from's acceptance tests, :350-364), with the
+// FP64 polish when the Jacobian is ill-conditioned: its t and texture
+// coordinate in double. The texel (lo_s, lo_t, w) and the ray's Q3 and 1/|d|
+// come from the leaf's setup; ray(o, d) gives the ray. flags gets
 // DMAP_HIT_FP64_LEAF | DMAP_HIT_POLISHED when the reported root is the FP64
-// Newton root. Kept out of line: it runs once per accepted root.
-static __device__ __noinline__ bool accept_root(const TriDev &T, const AssetDev &g, double lo_s, double lo_t, double w,
-                                         double Q3, double inv_dlen, v3 o, v3 d, double t_min, double t_max,
-                                         int64_t i, int64_t j, Root32 R, double polish_cond, hit64 &hit, int &flags,
-                                         int64_t &iters)
+// Newton root.
+template <class Ray>
+__device__ __forceinline__ bool judge_root(const TriDev &T, const AssetDev &g, const Leaf32 &L, const Ray &ray,
+                                           double t_min, double t_max, int64_t i, int64_t j, const Root32 &R,
+                                           double polish_cond, double &t, v2 &st, int &flags, int64_t &iters)
 {
-    double along = Q3 + (double)R.along_rel;
-    v2 st = V2(lo_s + w * (double)R.a, lo_t + w * (double)R.b);
+    double along = L.Q3 + (double)R.along_rel;
+    st = V2(L.lo_s + L.w * (double)R.a, L.lo_t + L.w * (double)R.b);
     if (along < 0.0 || !uv_inside(T, st))
         return false;
-    double t_hit = along * inv_dlen;
-    if (t_hit <= t_min || t_hit >= t_max)
+    t = along * L.inv_dlen;
+    if (t <= t_min || t >= t_max)
         return false;
+    flags = 0;
     float fro = R.J00 * R.J00 + R.J01 * R.J01 + R.J10 * R.J10 + R.J11 * R.J11;
     float det = fabsf(R.J00 * R.J11 - R.J01 * R.J10);
     if (fro > (float)polish_cond * det) { // cond(J) <= |J|_F^2 / |det J|
@@ -275,30 +287,38 @@ static __device__ __noinline__ bool accept_root(const TriDev &T, const AssetDev 
         // again from another start) or a farther one
         hit64 h;
         int64_t it = 0;
+        v3 o, d;
+        ray(o, d);
         bool ok = newton_from(T, g, o, d, t_min, INFINITY, i, j, st, h, it);
         iters += it;
         if (ok) {
             if (h.t >= t_max)
                 return false;
-            hit = h;
+            t = h.t;
+            st = h.st;
             flags = DMAP_HIT_FP64_LEAF | DMAP_HIT_POLISHED;
-            return true;
         }
     }
-    hit.t = t_hit;
-    hit.st = st;
-    hit.bary = tri_bary(T, st.x, st.y);
-    // the reference's normal, Su x Sv, at the root
-    nframe f = normal_frame_at(T, st.x, st.y);
-    double h;
-    v2 gh;
-    grid_h_grad(g, st.x, st.y, h, gh);
-    v3 Su = add3(add3(L3(T.e1), mul3(gh.x, f.N)), mul3(h, f.Nu));
-    v3 Sv = add3(add3(L3(T.e2), mul3(gh.y, f.N)), mul3(h, f.Nv));
-    hit.ng = normalized3(cross3(Su, Sv));
-    hit.i = i;
-    hit.j = j;
-    flags = 0;
+    return true;
+}
+
+// The same as a hit record, for a lane that searches alone. Kept out of
+// line: it runs once per accepted root.
+static __device__ __noinline__ bool accept_root(const TriDev &T, const AssetDev &g, const Leaf32 &L, v3 o, v3 d,
+                                                double t_min, double t_max, int64_t i, int64_t j, Root32 R,
+                                                double polish_cond, hit64 &hit, int &flags, int64_t &iters)
+{
+    double t;
+    v2 st;
+    int fl = 0;
+    auto ray = [&](v3 &ro, v3 &rd) {
+        ro = o;
+        rd = d;
+    };
+    if (!judge_root(T, g, L, ray, t_min, t_max, i, j, R, polish_cond, t, st, fl, iters))
+        return false;
+    flags = fl;
+    root_record(T, g, t, st, i, j, hit);
     return true;
 }
 
@@ -329,8 +349,7 @@ __device__ inline bool intersect_newton32(const TriDev &T, const TriDev32 &T32, 
             if (newton32(T, L, e.a, e.b, R, iters)) {
                 hit64 h;
                 int fl = 0;
-                if (accept_root(T, g, L.lo_s, L.lo_t, L.w, L.Q3, L.inv_dlen, o, d, t_min, t_max, i, j, R,
-                                polish_cond, h, fl, iters)) {
+                if (accept_root(T, g, L, o, d, t_min, t_max, i, j, R, polish_cond, h, fl, iters)) {
                     hit = h;
                     flags = fl;
                     t_max = h.t;

@@ -5,6 +5,8 @@
 // that must round the same way wherever they run are in walk32_exact.cu.
 #include "walk32.cuh"
 
+#include <algorithm>
+
 namespace dmapk
 {
 namespace w32
@@ -64,10 +66,12 @@ cudaError_t launch(Args a, const WaveScratch &ws, cudaStream_t stream)
     const int bps = a.opt.blocks_per_sm > 0              ? a.opt.blocks_per_sm
                     : a.n_tri > 32 * kMaskWords ? DMAP_WALK_TREE_MIN_BLOCKS
                                                          : DMAP_WALK_MIN_BLOCKS;
-    const int64_t need = (a.n + 31) / 32; // four lanes per ray
-    a.grid = sm_count() * bps;
-    if (need < a.grid)
-        a.grid = (int)need;
+    // four lanes per ray, but a batch that leaves quads idle spreads over the
+    // warps (one ray per warp where they suffice)
+    const int64_t need = (a.n + 3) / 4;
+    a.grid = (int)std::min<int64_t>(sm_count() * bps, need);
+    a.filter_grid = (int)std::min<int64_t>(sm_count() * 8, (a.n + 31) / 32);
+    a.leaf_grid = (int)std::min<int64_t>(sm_count() * kLeafBlocks, (a.n + 1) / 2);
     a.states = ws.state;
     a.leaves = ws.leaves;
     a.counters = ws.counters;
@@ -80,12 +84,8 @@ cudaError_t launch(Args a, const WaveScratch &ws, cudaStream_t stream)
                 return e;
             return simple_rerun<R, H, Fp>(a, stream);
         }
-        if ((e = walk_round(a, q_in, rd, stream)) != cudaSuccess ||
-            (e = filter<R>(a, rd, stream)) != cudaSuccess)
-            return e;
-        e = a.opt.leaf_precision == 1 ? leaf32<R, H, Fp>(a, rd, q_out, stream) // the FP32 certified leaf
-                                      : leaf64<R, H, Fp>(a, rd, q_out, stream);
-        if (e != cudaSuccess)
+        if ((e = walk_round(a, q_in, rd, stream)) != cudaSuccess || (e = filter(a, rd, stream)) != cudaSuccess ||
+            (e = leaves(a, rd, q_out, stream)) != cudaSuccess)
             return e;
     }
     return cudaSuccess;
@@ -115,7 +115,7 @@ cudaError_t launch_walk32(const dmapdev::TriDev32 *t32, const dmapdev::TriDev *t
     if (n <= 0)
         return cudaSuccess;
     const w32::Args a = {t32, t64, n_tri, assets, rays, n, opt, hits, stats, status, nullptr, nullptr, nullptr,
-                         nullptr, 0};
+                         nullptr, 0, 0, 0};
     const bool r64 = opt.ray_dtype == 2, h64 = opt.hit_dtype == 2;
     if (r64 && h64)
         return w32::launch<double, dmapdev::Hit64, double>(a, ws, stream);

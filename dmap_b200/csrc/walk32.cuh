@@ -49,6 +49,7 @@
 #include "f32_node.cuh"
 #include "bvh.cuh"
 #include "leaf32.cuh"
+#include "leaf_quad.cuh"
 #include "order.cuh"
 #include "filter.cuh"
 #include "instance.cuh"
@@ -60,19 +61,16 @@ using dmapdev::AssetDev;
 using dmapdev::TriDev;
 using dmapdev::TriDev32;
 
-// Resident 128-thread CTAs per SM the walk and leaf kernels are compiled for
-// (register budget: 65536 / (128 x blocks) per thread). The walk rounds over
-// the per-ray candidate mask (scenes of up to 256 triangles) take 4 (119
-// registers, no spills: faster than 5 at 96 registers with spills); over the
-// triangle tree, whose candidate buffer lives in local memory either way, 5.
+// Resident 128-thread CTAs per SM the walk is compiled for (register budget:
+// 65536 / (128 x blocks) per thread). The walk rounds over the per-ray
+// candidate mask (scenes of up to 256 triangles) take 4 (112 registers, no
+// spills); over the triangle tree, whose candidate buffer lives in local
+// memory either way, 5.
 #ifndef DMAP_WALK_MIN_BLOCKS
 #define DMAP_WALK_MIN_BLOCKS 4
 #endif
 #ifndef DMAP_WALK_TREE_MIN_BLOCKS
 #define DMAP_WALK_TREE_MIN_BLOCKS 5
-#endif
-#ifndef DMAP_LEAF_MIN_BLOCKS
-#define DMAP_LEAF_MIN_BLOCKS 1
 #endif
 // Node tests a ray may run past its first collected leaf before it parks.
 #ifndef DMAP_STALE_CAP
@@ -405,10 +403,12 @@ struct RayState
     int cl, ci, cj;
     int nah, lah, pad;
     unsigned long long todo[2], dom[2];
-    unsigned long long mask[4]; // per lane of the ray's four
-    // scenes of more than 256 triangles: the buffered candidates, kept
-    // across parks so a resumed ray does not walk the tree again
-    d32::NearBuf buf;
+    union {
+        unsigned long long mask[4]; // per lane of the ray's four
+        // scenes of more than 256 triangles: the buffered candidates, kept
+        // across parks so a resumed ray does not walk the tree again
+        d32::NearBuf buf;
+    };
 };
 // Up to kCollect consecutive leaves of one triangle's walk, in walk order.
 // The walk goes on past a leaf with the t_max it has (it cannot know the
@@ -424,7 +424,8 @@ constexpr int kCollect = 4; // leaf slots of a job
 static_assert(DMAP_COLLECT >= 1 && DMAP_COLLECT <= kCollect, "leaf slots");
 struct LeafJob
 {
-    int ray, tri, n, pad;
+    int ray, tri, n;
+    int keep; // the cells the FP64 node test admits, a bit each (wave_filter)
     int i[kCollect], j[kCollect];
 };
 // RayState.flags
@@ -454,6 +455,80 @@ __device__ __forceinline__ void check_crossing(const dmapk::QueryOpts &opt, cons
 __device__ __forceinline__ unsigned long long *round_ctr(unsigned long long *c, int round, int k)
 {
     return c + 4 * round + k;
+}
+
+// A leaf cell the last walk reached, by the four lanes of its ray's quad: the
+// cell's FP64 node test, then the certified leaf in the query's precision.
+// A nearer root is stored as the ray's hit; returns the ray's t_max.
+template <class P, bool ST>
+__device__ __noinline__ double quad_leaf(const TriDev32 &T32, const TriDev &T, const AssetDev *assets, const void *rays,
+                                         int ray, int tri, double t_max, int i, int j, const dmapk::QueryOpts &opt,
+                                         void *hits, double *stack_mem, unsigned long long *ctr, int *rerun, int &flags,
+                                         int64_t *stl)
+{
+    const int lane = threadIdx.x & 31;
+    const lq::Quad Q = {0xfu << (lane & 28), lane & 28, lane & 3};
+    const AssetDev &g = assets[T.asset];
+    typename P::Ent *stack = reinterpret_cast<typename P::Ent *>(stack_mem);
+    double o[3], d[3], t_min, t_ray;
+    load_ray(rays, opt.ray_dtype, ray, o, d, t_min, t_ray);
+    if (T.inst) {
+        // an instanced triangle meets the ray in its object space (instance.cuh)
+        double oo[3], od[3];
+        dmapdev::object_ray(opt.inst_xf + dmapdev::kInstDoubles * (T.inst - 1), o, d, oo, od);
+        for (int a = 0; a < 3; ++a) {
+            o[a] = oo[a];
+            d[a] = od[a];
+        }
+    }
+    const d64::v3 O = d64::V3(o[0], o[1], o[2]), D = d64::V3(d[0], d[1], d[2]);
+    if (!d64::leaf_cell_admitted(T, g, O, D, t_min, t_max, i, j, opt))
+        return t_max;
+    typename P::Bound L;
+    P::setup(T, g, O, D, i, j, L);
+    auto ray_of = [&](d64::v3 &ro, d64::v3 &rd) {
+        ro = O;
+        rd = D;
+    };
+    // the last root taken, in the lane that took it
+    lq::Found best;
+    double mine = -INFINITY;
+    auto on_root = [&](const lq::Found &f) {
+        best = f;
+        mine = f.t;
+    };
+    const double t_start = t_max;
+    typename P::Ent e = lq::root_entry<P>();
+    int sp = 0;
+    int64_t subs = 0, iters = 0;
+    do {
+        lq::Child<P> c;
+        lq::bound_children<P>(Q, e, T32, T, L, t_min, t_max, c);
+        if (ST)
+            subs += 4;
+        if (e.depth + 1 < lq::kDepth)
+            lq::push_children<P>(Q, c, e.depth + 1, stack, sp);
+        else if (c.n > 0 && lq::newton_children<P, ST>(Q, c, T, g, L, ray_of, t_min, t_max, i, j, opt.polish_cond,
+                                                       opt.mode == 1, iters, on_root))
+            break;
+    } while (lq::pop<P>(stack, sp, t_max, e));
+    if (mine == t_max && t_max < t_start) {
+        d64::hit64 h;
+        d64::root_record(T, g, best.t, best.st, i, j, h);
+        if (T.inst)
+            dmapdev::world_normal(opt.inst_xf + dmapdev::kInstDoubles * (T.inst - 1), h.ng);
+        store_hit(hits, opt.hit_dtype, ray, true, h, tri, best.flags | ((flags & kCapped) ? DMAP_HIT_CAPPED : 0));
+        check_crossing(opt, T, tri, h, ray, flags, ctr, rerun);
+    }
+    __syncwarp(Q.mask);
+    flags = (int)__reduce_or_sync(Q.mask, (unsigned)flags);
+    if (ST) {
+        iters += __shfl_xor_sync(Q.mask, iters, 1);
+        iters += __shfl_xor_sync(Q.mask, iters, 2);
+        stl[DMAP_ST_SUB] += subs;
+        stl[DMAP_ST_NEWTON] += iters;
+    }
+    return t_max;
 }
 
 // Four lanes walk one ray (a quad; eight rays per warp), so that the four
@@ -515,6 +590,8 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
         }
         __syncthreads();
     }
+    // the last walk: the leaf search's stacks, per quad
+    __shared__ double s_stack[INLINE_LEAF ? 32 : 1][INLINE_LEAF ? lq::kStack * sizeof(lq::P64::Ent) / 8 : 1];
     auto box32 = [&](int t, float *lo, float *hi) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -594,7 +671,6 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
             job.ray = ray;
             job.tri = tri;
             job.n = nl;
-            job.pad = 0;
         }
         job.i[sub] = li;
         job.j[sub] = lj;
@@ -982,36 +1058,26 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
 
         if (INLINE_LEAF) {
             // the last round: the few remaining rays finish here
-            int got = 0;
-            if (leaf && sub == 0) {
-                double o[3], d[3], t_min, t_ray;
-                load_ray(rays, opt.ray_dtype, ray, o, d, t_min, t_ray);
-                d64::hit64 lh;
-                int lf = 0;
-                if (leaf_cell(tris32[tri], tris64[tri], assets[tris32[tri].asset], o, d, t_min, t_max, cur.i, cur.j, lh,
-                              lf, ST ? stl : nullptr, opt) &&
-                    lh.t < t_max) {
-                    t_max = lh.t;
-                    got = 1;
-                    store_hit(hits, opt.hit_dtype, ray, true, lh, tri, lf | ((flags & kCapped) ? DMAP_HIT_CAPPED : 0));
-                    check_crossing(opt, tris64[tri], tri, lh, ray, flags, ctr, rerun);
+            if (leaf) {
+                const double t_old = t_max;
+                t_max = opt.leaf_precision == 1
+                            ? quad_leaf<lq::P32, ST>(tris32[tri], tris64[tri], assets, rays, ray, tri, t_max, cur.i, cur.j,
+                                                     opt, hits, s_stack[threadIdx.x >> 2], ctr, rerun, flags, stl)
+                            : quad_leaf<lq::P64, ST>(tris32[tri], tris64[tri], assets, rays, ray, tri, t_max, cur.i, cur.j,
+                                                     opt, hits, s_stack[threadIdx.x >> 2], ctr, rerun, flags, stl);
+                if (t_max < t_old) {
+                    tmax_f = __double2float_ru(t_max);
+                    best_tri = tri;
+                    flags |= kFoundInTri;
+                    nah = lah = 0;
+                    stale = ~0u;
+                    if (opt.mode == 1) {
+                        flush_stats();
+                        phase = NEED;
+                    }
                 }
             }
             __syncwarp();
-            got = __shfl_sync(FULL, got, lead);
-            t_max = __shfl_sync(FULL, t_max, lead);
-            flags = __shfl_sync(FULL, flags, lead);
-            if (leaf && got) {
-                tmax_f = __double2float_ru(t_max);
-                best_tri = tri;
-                flags |= kFoundInTri;
-                nah = lah = 0;
-                stale = ~0u;
-                if (opt.mode == 1) {
-                    flush_stats();
-                    phase = NEED;
-                }
-            }
         }
 
         // 3b. the group's cells, one per lane, all quads together
@@ -1048,399 +1114,336 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
 
 // The leaf cells of a round's jobs through the reference's own node test in
 // double (node_bounds.cpp:83-211 at level 0, the node computed from the
-// grid): the FP32 walk, widened by its roundings, reaches more leaf cells
-// than the FP64 walk, and a cell the FP64 walk rejects has no leaf there.
-// The ray's t_max is the one it parked with; earlier leaves of the same job
-// can only shrink it, so a cell kept here may still be rejected by the FP64
-// walk at that point, and its search then finds nothing the reference
-// would not. Cells are compacted in walk order; a job may end up empty.
-// Kept apart from the leaf kernel so that kernel's code stays small.
-template <typename R>
+// grid), a lane per cell: the FP32 walk, widened by its roundings, reaches
+// more leaf cells than the FP64 walk, and a cell the FP64 walk rejects has no
+// leaf there. The ray's t_max is the one it parked with; earlier leaves of
+// the same job can only shrink it, so a cell kept here may still be rejected
+// by the FP64 walk at that point, and its search then finds nothing the
+// reference would not. Kept apart from the leaf kernel so that kernel's code
+// stays small.
 __global__ void __launch_bounds__(128)
-    wave_filter(const TriDev *__restrict__ tris64, const AssetDev *__restrict__ assets, const R *__restrict__ rays,
+    wave_filter(const TriDev *__restrict__ tris64, const AssetDev *__restrict__ assets, const void *__restrict__ rays,
                 dmapk::QueryOpts opt, const RayState *__restrict__ states, LeafJob *__restrict__ q_leaf, int round,
                 const unsigned long long *ctr)
 {
-    const unsigned long long count = *round_ctr(const_cast<unsigned long long *>(ctr), round, 1);
+    const unsigned long long count = 4ull * *round_ctr(const_cast<unsigned long long *>(ctr), round, 1);
+    const int lead = threadIdx.x & 28, sub = threadIdx.x & 3;
     for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; k < count;
          k += (unsigned long long)gridDim.x * blockDim.x) {
-        LeafJob job = q_leaf[k];
-        double o[3], d[3], t_min, t_max;
-        load_ray(rays, job.ray, o, d, t_min, t_max);
-        t_max = states[job.ray].t_max;
-        const TriDev &T = tris64[job.tri];
-        const AssetDev &g = assets[T.asset];
-        if (T.inst) {
-            double oo[3], od[3];
-            dmapdev::object_ray(opt.inst_xf + dmapdev::kInstDoubles * (T.inst - 1), o, d, oo, od);
-            for (int a = 0; a < 3; ++a) {
-                o[a] = oo[a];
-                d[a] = od[a];
-            }
+        LeafJob &job = q_leaf[k >> 2];
+        bool admitted = false;
+        if (sub < job.n) {
+            double o[3], d[3], oo[3], od[3], t_min, t_max;
+            load_ray(rays, opt.ray_dtype, job.ray, o, d, t_min, t_max);
+            t_max = states[job.ray].t_max;
+            const TriDev &T = tris64[job.tri];
+            dmapdev::ray_for(opt.inst_xf, T.inst, o, d, oo, od);
+            admitted = d64::leaf_cell_admitted(T, assets[T.asset], d64::V3(oo[0], oo[1], oo[2]),
+                                               d64::V3(od[0], od[1], od[2]), t_min, t_max, job.i[sub], job.j[sub], opt);
         }
-        d64::tray r = d64::tangent_ray64(T, d64::V3(o[0], o[1], o[2]), d64::V3(d[0], d[1], d[2]), t_min, t_max);
-        int m = 0;
-#pragma unroll 1
-        for (int q = 0; q < job.n; ++q) {
-            if (d64::leaf_cell_admitted(T, g, r, job.i[q], job.j[q], opt)) {
-                job.i[m] = job.i[q];
-                job.j[m] = job.j[q];
-                ++m;
-            }
-        }
-        if (m != job.n) {
-            job.n = m;
-            q_leaf[k] = job;
-        }
+        const unsigned quad = 0xfu << lead;
+        __syncwarp(quad);
+        const unsigned keep = __ballot_sync(quad, admitted);
+        if (sub == 0)
+            job.keep = (int)((keep >> lead) & 15u);
     }
 }
 
-// The parked leaves of a round (the certified leaf, d64::intersect_newton,
-// displaced_intersector.cpp:239-323). Each lane holds one job at a time and
-// takes the next one as soon as its own is done, so a warp's lanes stay busy
-// however long their leaves run. A step of the loop runs, for the lanes that
-// need it: the leaf setup, one sub-square expansion (four bounds, the sort,
-// the push) or one Newton run, with the warp reconverged between blocks.
-// Each lane's search is intersect_newton's, in the same order with the same
-// arithmetic, so each ray's result equals it bit for bit. A ray whose walk
-// has cells left goes back to the resume queue.
-template <bool ST, typename R, typename H, typename Fp>
-__global__ void __launch_bounds__(128, DMAP_LEAF_MIN_BLOCKS)
-    wave_leaf(const TriDev *__restrict__ tris64, const AssetDev *__restrict__ assets, const R *__restrict__ rays,
-              dmapk::QueryOpts opt, H *__restrict__ hits, int64_t *__restrict__ stats, RayState *__restrict__ states,
+// The parked leaves of a round, a quad per job: the cells the filter kept are
+// searched in walk order, all four lanes together (leaf_quad.cuh), one entry
+// per step, quads at the same kind of step side by side. A ray whose walk has
+// cells left goes back to the resume queue.
+//
+// The leaf setups (some 800 double operations each) are made by the warp for
+// eight jobs at a time, a lane per cell, ahead of the quads that take them:
+// shared memory holds the setups of the cells in work and of those made
+// ready, up to 32 a warp, and the search reads them there (in registers they
+// spilled). Newton runs wait until DMAP_NEWTON_QUADS of a warp's quads have
+// some, and the hit records of the roots found (some 200 double operations
+// behind two chains of loads) until the warp has a batch of them. Each quad
+// making its own setups and records as they came, with one or two of the
+// warp's lanes in it, spent most of the kernel there. Leaf rounds of 2.80M
+// rays on the sphere of 96 x 2048^2 maps: a lane per job 9.1 ms, quads 19.7,
+// with batched setups 15.1, batched Newton runs and records 10.0, setups in
+// shared memory 8.1; of 20,011 rays on 512^2 maps 0.72 -> 0.27 ms. The kernel
+// issues in 22% of its cycles at 3 warps per scheduler, half of its stalls
+// instruction fetch.
+// Resident CTAs per SM the leaf kernels are compiled for: 6 for the FP32 leaf
+// (168 registers; 5, 7 and 8 are 1-12% slower), 4 for the FP64 leaf.
+#ifndef DMAP_LEAF32_MIN_BLOCKS
+#define DMAP_LEAF32_MIN_BLOCKS 6
+#endif
+#ifndef DMAP_LEAF_MIN_BLOCKS
+#define DMAP_LEAF_MIN_BLOCKS 4
+#endif
+// Quads of a warp with Newton runs waiting before the warp makes them.
+#ifndef DMAP_NEWTON_QUADS
+#define DMAP_NEWTON_QUADS 4
+#endif
+constexpr int kLeafThreads = 64;
+constexpr int kLeafBlocks = DMAP_LEAF32_MIN_BLOCKS;
+template <bool ST, class P>
+__global__ void __launch_bounds__(kLeafThreads,
+                                  sizeof(typename P::Real) == 4 ? DMAP_LEAF32_MIN_BLOCKS : DMAP_LEAF_MIN_BLOCKS)
+    wave_leaf(const TriDev32 *__restrict__ tris32, const TriDev *__restrict__ tris64,
+              const AssetDev *__restrict__ assets, const void *__restrict__ rays, dmapk::QueryOpts opt,
+              void *__restrict__ hits, int64_t *__restrict__ stats, RayState *__restrict__ states,
               const LeafJob *__restrict__ q_leaf, int round, int *__restrict__ q_out, unsigned long long *ctr,
               int *__restrict__ rerun)
 {
     using namespace d64;
-    constexpr int kDepth = 5; // subdivision_depth
-    enum : int { NEED = 0, SETUP = 1, SEARCH = 2, DONE = 3 };
-    const int lane = threadIdx.x & 31;
+    typedef typename P::Ent Ent;
+    typedef typename P::Bound Bound;
+    enum : int { NEED = 0, SEARCH = 1, NEWTON = 2, DONE = 3 };
+    constexpr int kSlots = 16; // jobs per warp: eight in work, eight ready
+    constexpr int kRecs = 32;  // leaf setups per warp
+    constexpr int kReps = 16;  // hit records per warp still to be made
+    __shared__ Bound s_rec[kLeafThreads / 32][kRecs];
+    struct Slot { int ray, tri, keep, i[kCollect], j[kCollect]; unsigned char rec[kCollect]; };
+    __shared__ Slot s_job[kLeafThreads / 32][kSlots];
+    __shared__ Ent s_stack[kLeafThreads / 4][lq::kStack];
+    // the root each quad's job holds, and the roots of finished jobs whose
+    // records are still to be made
+    struct Rep { double t, s, v; int ray, tri, i, j, flags, pad; };
+    __shared__ Rep s_best[kLeafThreads / 4], s_rep[kLeafThreads / 32][kReps];
+    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5, qi = threadIdx.x >> 2;
+    const lq::Quad Q = {0xfu << (lane & 28), lane & 28, lane & 3};
     const unsigned long long count = *round_ctr(ctr, round, 1);
     unsigned long long *fetch = round_ctr(ctr, round, 2);
-    int phase = NEED;
-    unsigned long long item = 0;
-    int ray = 0, tri = 0, n_leaves = 0, q = 0, li = 0, lj = 0, sp = 0;
-    bool first = false, answered = false;
+    // as the walk: a round of few jobs spreads them over all warps
+    const unsigned long long warps = (unsigned long long)gridDim.x * (kLeafThreads / 32);
+    const int batch = (int)min(8ull, (count + warps - 1ull) / warps);
+    int phase = (lane >> 2) < batch ? NEED : DONE;
+    unsigned long long next = 0, last = 0; // items of the queue this warp holds and has not set up
+    bool more = batch > 0;                 // items may be left in the queue
+    unsigned ready = 0u;                   // slots with a job set up and not yet taken
+    unsigned recs = 0u;                    // setups in use
+    int slot = 0, rec = -1;                // the quad's job, the setup of its cell
+    int ray = 0, tri = 0, ci = 0, cj = 0, sp = 0;
+    unsigned keep = 0u; // the job's cells not yet searched
+    bool answered = false, found = false;
+    int n_rep = 0;
     double t_min = 0.0, t_max = 0.0;
-    v3 O = V3(0.0, 0.0, 0.0), D = O;
-    leafbound L;
-    leafent stack[4 * kDepth + 4];
+    lq::Child<P> c;
+    c.pass = false;
+    c.n = 0;
     int64_t subs = 0, iters = 0;
 
+    // the job's ray, in its triangle's space
+    auto ray_of = [&](v3 &O, v3 &D) {
+        double o[3], d[3], t0, t1;
+        load_ray(rays, opt.ray_dtype, ray, o, d, t0, t1);
+        const int inst = tris64[tri].inst;
+        if (inst) {
+            double oo[3], od[3];
+            dmapdev::object_ray(opt.inst_xf + dmapdev::kInstDoubles * (inst - 1), o, d, oo, od);
+            O = V3(oo[0], oo[1], oo[2]);
+            D = V3(od[0], od[1], od[2]);
+        } else {
+            O = V3(o[0], o[1], o[2]);
+            D = V3(d[0], d[1], d[2]);
+        }
+    };
+    // the records of the roots found, a lane per root
+    auto report = [&]() {
+        __syncwarp();
+        if (lane < n_rep) {
+            const Rep &r = s_rep[wi][lane];
+            const TriDev &T = tris64[r.tri];
+            hit64 h;
+            root_record(T, assets[T.asset], r.t, V2(r.s, r.v), r.i, r.j, h);
+            if (T.inst)
+                dmapdev::world_normal(opt.inst_xf + dmapdev::kInstDoubles * (T.inst - 1), h.ng);
+            RayState &s = states[r.ray];
+            store_hit(hits, opt.hit_dtype, r.ray, true, h, r.tri, r.flags | ((s.flags & kCapped) ? DMAP_HIT_CAPPED : 0));
+            check_crossing(opt, T, r.tri, h, r.ray, s.flags, ctr, rerun);
+        }
+        n_rep = 0;
+        __syncwarp();
+    };
+
     for (;;) {
-        // lanes without a job take the next ones, one atomic per warp
-        unsigned need = __ballot_sync(FULL, phase == NEED);
-        if (need) {
-            int leader = __ffs(need) - 1;
-            unsigned long long base = 0;
-            if (lane == leader)
-                base = atomicAdd(fetch, (unsigned long long)__popc(need));
-            base = __shfl_sync(FULL, base, leader);
-            if (phase == NEED) {
-                item = base + (unsigned long long)__popc(need & ((1u << lane) - 1u));
-                if (item >= count) {
-                    phase = DONE;
-                } else {
-                    const LeafJob &J = q_leaf[item];
+        // quads without a job take one that is ready; when none is, the warp
+        // sets up the next eight of the queue, a lane per cell
+        unsigned need;
+        while ((need = __ballot_sync(FULL, phase == NEED) & 0x11111111u) != 0u) {
+            if (ready) {
+                const int k = __popc(need & ((1u << Q.lead) - 1u)), have = __popc(ready), want = __popc(need);
+                if (phase == NEED && k < have) {
+                    slot = (int)__fns(ready, 0, k + 1);
+                    const Slot &J = s_job[wi][slot];
                     ray = J.ray;
                     tri = J.tri;
-                    n_leaves = J.n;
-                    q = 0;
-                    if (n_leaves == 0) {
-                        // the filter rejected every cell of the job: the walk goes on
-                        unsigned long long slot = atomicAdd(round_ctr(ctr, round, 3), 1ull);
-                        q_out[slot] = ray;
-                    } else {
-                        double o[3], d[3];
-                        load_ray(rays, ray, o, d, t_min, t_max);
-                        if (tris64[tri].inst) {
-                            double oo[3], od[3];
-                            dmapdev::object_ray(opt.inst_xf + dmapdev::kInstDoubles * (tris64[tri].inst - 1), o, d,
-                                                oo, od);
-                            for (int a = 0; a < 3; ++a) {
-                                o[a] = oo[a];
-                                d[a] = od[a];
-                            }
-                        }
-                        O = V3(o[0], o[1], o[2]);
-                        D = V3(d[0], d[1], d[2]);
-                        t_max = states[ray].t_max;
-                        answered = false;
-                        subs = iters = 0;
-                        phase = SETUP;
-                    }
+                    keep = (unsigned)J.keep;
+                    double o[3], d[3];
+                    load_ray(rays, opt.ray_dtype, ray, o, d, t_min, t_max);
+                    t_max = states[ray].t_max;
+                    sp = 0;
+                    subs = iters = 0;
+                    answered = found = false;
+                    phase = SEARCH;
+                }
+                for (int q = 0; q < want; ++q)
+                    ready &= ready - 1u;
+                __syncwarp();
+                continue;
+            }
+            if (next == last) {
+                if (!more) {
+                    if (phase == NEED)
+                        phase = DONE;
+                    break;
+                }
+                if (lane == 0)
+                    next = atomicAdd(fetch, (unsigned long long)batch);
+                next = __shfl_sync(FULL, next, 0);
+                last = min(next + batch, count);
+                more = last < count;
+                if (next >= last) {
+                    next = last = 0;
+                    continue;
                 }
             }
+            // the next jobs whose cells the free setups hold: a lane per cell
+            const unsigned long long item = next + (lane >> 2);
+            unsigned cells = 0u;
+            int jr = 0, jt = 0, li = 0, lj = 0;
+            if (item < last) {
+                const LeafJob &J = q_leaf[item];
+                cells = (unsigned)J.keep;
+                jr = J.ray;
+                jt = J.tri;
+                li = J.i[Q.sub];
+                lj = J.j[Q.sub];
+            }
+            const unsigned kept = __ballot_sync(FULL, (cells >> Q.sub) & 1u);
+            const bool fits = item < last && __popc(kept & (unsigned)((16ull << Q.lead) - 1ull)) <= kRecs - __popc(recs);
+            const unsigned took = __ballot_sync(FULL, fits) & 0x11111111u;
+            if (!took)
+                break; // the jobs in work hold them
+            next += __popc(took);
+            // the slots no quad's job is in
+            const unsigned taken = __reduce_or_sync(FULL, phase == SEARCH || phase == NEWTON ? 1u << slot : 0u);
+            const int to = (int)__fns(~taken, 0, (lane >> 2) + 1);
+            unsigned mine = 0u;
+            if (fits) {
+                Slot &S = s_job[wi][to];
+                if (Q.sub == 0) {
+                    S.ray = jr;
+                    S.tri = jt;
+                    S.keep = (int)cells;
+                    if (!cells) // the filter rejected every cell of the job: the walk goes on
+                        q_out[atomicAdd(round_ctr(ctr, round, 3), 1ull)] = jr;
+                }
+                S.i[Q.sub] = li;
+                S.j[Q.sub] = lj;
+                if ((cells >> Q.sub) & 1u) {
+                    const int at = (int)__fns(~recs, 0, __popc(kept & ((1u << lane) - 1u)) + 1);
+                    S.rec[Q.sub] = (unsigned char)at;
+                    mine = 1u << at;
+                    double o[3], d[3], oo[3], od[3], t0, t1;
+                    load_ray(rays, opt.ray_dtype, jr, o, d, t0, t1);
+                    const TriDev &T = tris64[jt];
+                    dmapdev::ray_for(opt.inst_xf, T.inst, o, d, oo, od);
+                    P::setup(T, assets[T.asset], V3(oo[0], oo[1], oo[2]), V3(od[0], od[1], od[2]), li, lj, s_rec[wi][at]);
+                }
+            }
+            __syncwarp();
+            recs |= __reduce_or_sync(FULL, mine);
+            ready = __reduce_or_sync(FULL, fits && cells ? 1u << to : 0u);
         }
         if (__all_sync(FULL, phase == DONE))
             break;
-        const TriDev &T = tris64[tri];
-        const AssetDev &g = assets[T.asset];
-        // leaf q of the job (a cell wave_filter kept): the texel's corners,
-        // its normal form and the ray's plane basis (:239-264)
-        if (phase == SETUP) {
-            li = q_leaf[item].i[q];
-            lj = q_leaf[item].j[q];
-            sp = 0;
-            phase = SEARCH;
-            L.w = cell_width(g, 0);
-            L.lo = {li * L.w, lj * L.w};
-            L.h00 = grid_h(g, L.lo.x, L.lo.y);
-            L.h10 = grid_h(g, L.lo.x + L.w, L.lo.y);
-            L.h01 = grid_h(g, L.lo.x, L.lo.y + L.w);
-            L.h11 = grid_h(g, L.lo.x + L.w, L.lo.y + L.w);
-            v2 c = add2(L.lo, V2(0.5 * L.w, 0.5 * L.w));
-            double hw = 0.5 * L.w;
-            L.N_hat = AF3(add3(add3(L3(T.m0), mul3(c.x, L3(T.Mu))), mul3(c.y, L3(T.Mv))), mul3(hw, L3(T.Mu)),
-                          mul3(hw, L3(T.Mv)));
-            normalize(L.N_hat);
-            L.o = O;
-            L.d_len = norm3(D);
-            L.dn = div3(D, L.d_len);
-            plane_basis(L.dn, L.d1, L.d2);
-            stack[sp++] = {0.5, 0.5, -INFINITY, 0};
-            first = true;
-        }
-        // the next live entry of the search (a pop is a call of search_leaf;
-        // an entry at or beyond t_max is the sorted loop's break)
-        bool expand = false, newton = false;
-        leafent e = {0.0, 0.0, 0.0, 0};
+        // the next entry of the search, the next cell's root, or the job is done
+        bool have = false;
+        unsigned done = 0u;
+        Ent e = lq::root_entry<P>();
         if (phase == SEARCH) {
-            while (sp > 0) {
-                e = stack[--sp];
-                if (first || e.t_lo < t_max) {
-                    first = false;
-                    newton = e.depth == kDepth;
-                    expand = !newton;
-                    break;
-                }
+            have = lq::pop<P>(s_stack[qi], sp, t_max, e);
+            if (!have && rec >= 0) {
+                done = 1u << rec; // the cell's setup is free again
+                rec = -1;
             }
-            if (!expand && !newton) {
-                // the leaf is done; the next of the job, or the job is done
-                if (++q < n_leaves && !answered) {
-                    phase = SETUP;
-                } else {
+            if (answered) // the cells left are not searched
+                for (; keep; keep &= keep - 1u)
+                    done |= 1u << s_job[wi][slot].rec[__ffs(keep) - 1];
+            if (!have && keep) {
+                const int q = __ffs(keep) - 1;
+                keep &= keep - 1u;
+                ci = s_job[wi][slot].i[q];
+                cj = s_job[wi][slot].j[q];
+                rec = s_job[wi][slot].rec[q];
+                e = lq::root_entry<P>();
+                have = true;
+            }
+            if (!have) {
+                if (ST) {
+                    iters += __shfl_xor_sync(Q.mask, iters, 1);
+                    iters += __shfl_xor_sync(Q.mask, iters, 2);
+                }
+                if (Q.sub == 0) {
                     if (ST) {
                         stats[DMAP_ST_N * (int64_t)ray + DMAP_ST_SUB] += subs;
                         stats[DMAP_ST_N * (int64_t)ray + DMAP_ST_NEWTON] += iters;
                     }
-                    if (!answered) {
-                        unsigned long long slot = atomicAdd(round_ctr(ctr, round, 3), 1ull);
-                        q_out[slot] = ray;
+                    if (found) {
+                        RayState &s = states[ray];
+                        s.t_max = t_max;
+                        s.best_tri = tri;
+                        s.flags |= kFoundInTri | kShrunk;
+                        s.nah = s.lah = 0;
                     }
-                    phase = NEED;
+                    if (!answered)
+                        q_out[atomicAdd(round_ctr(ctr, round, 3), 1ull)] = ray;
                 }
+                phase = NEED;
             }
         }
-        __syncwarp();
-        if (expand) {
-            double r = 0.5 * ldexp(0.5, -e.depth);
-            leafent ch[4];
-            int n = 0;
-#pragma unroll 1
-            for (int k = 0; k < 4; ++k) {
-                double ca = e.a + ((k & 1) ? r : -r), cb = e.b + ((k & 2) ? r : -r), t_lo;
-                ++subs;
-                if (sub_square_bound(T, L, ca, cb, r, t_min, t_max, t_lo))
-                    ch[n++] = {ca, cb, t_lo, e.depth + 1};
+        recs &= ~__reduce_or_sync(FULL, done);
+        // finished jobs' roots join the batch
+        const unsigned fin = __ballot_sync(FULL, phase == NEED && found) & 0x11111111u;
+        if (fin) {
+            if (phase == NEED && found) {
+                if (Q.sub == 0)
+                    s_rep[wi][n_rep + __popc(fin & ((1u << Q.lead) - 1u))] = s_best[qi];
+                found = false;
             }
-            for (int p = 1; p < n; ++p)
-                for (int k = p; k > 0 && ch[k].t_lo < ch[k - 1].t_lo; --k) {
-                    leafent x = ch[k];
-                    ch[k] = ch[k - 1];
-                    ch[k - 1] = x;
-                }
-            for (int k = n - 1; k >= 0; --k)
-                stack[sp++] = ch[k];
+            n_rep += __popc(fin);
+            if (n_rep > kReps - 8)
+                report();
+        }
+        if (have) {
+            const TriDev &T = tris64[tri];
+            lq::bound_children<P>(Q, e, tris32[tri], T, s_rec[wi][rec], t_min, t_max, c);
+            if (ST)
+                subs += 4;
+            if (e.depth + 1 < lq::kDepth)
+                lq::push_children<P>(Q, c, e.depth + 1, s_stack[qi], sp);
+            else if (c.n > 0)
+                phase = NEWTON;
         }
         __syncwarp();
-        if (newton) {
-            hit64 h;
-            if (newton_from(T, g, O, D, t_min, t_max, li, lj, add2(L.lo, mul2(L.w, V2(e.a, e.b))), h, iters)) {
-                // a nearer root of this leaf (each later one is nearer still)
-                t_max = h.t;
-                RayState &s = states[ray];
-                s.t_max = h.t;
-                s.best_tri = tri;
-                s.flags |= kFoundInTri | kShrunk;
-                s.nah = s.lah = 0;
-                if (tris64[tri].inst)
-                    dmapdev::world_normal(opt.inst_xf + dmapdev::kInstDoubles * (tris64[tri].inst - 1), h.ng);
-                store_hit<H, Fp>(hits, ray, true, h, tri,
-                                 DMAP_HIT_FP64_LEAF | ((s.flags & kCapped) ? DMAP_HIT_CAPPED : 0));
-                check_crossing(opt, tris64[tri], tri, h, ray, s.flags, ctr, rerun);
-                if (opt.mode == 1) { // occlusion: any hit answers the query
+        const unsigned wait = __ballot_sync(FULL, phase == NEWTON) & 0x11111111u;
+        if (__popc(wait) >= DMAP_NEWTON_QUADS || (wait && !__any_sync(FULL, phase == SEARCH))) {
+            if (phase == NEWTON) {
+                const TriDev &T = tris64[tri];
+                auto on_root = [&](const lq::Found &f) {
+                    s_best[qi] = {f.t, f.st.x, f.st.y, ray, tri, ci, cj, f.flags, 0};
+                };
+                const double t_old = t_max;
+                phase = SEARCH;
+                if (lq::newton_children<P, ST>(Q, c, T, assets[T.asset], s_rec[wi][rec], ray_of, t_min, t_max, ci, cj, opt.polish_cond,
+                                               opt.mode == 1, iters, on_root)) {
+                    // occlusion: any hit answers the query
                     answered = true;
                     sp = 0;
                 }
+                found = found || t_max < t_old;
             }
+            __syncwarp();
         }
-        __syncwarp();
     }
-}
-
-// The parked leaves of a round with the FP32 certified leaf (leaf32.cuh):
-// wave_leaf's schedule (one job per lane, a lane takes the next job when its
-// own is done, one search step per loop iteration) over the FP32 leaf state.
-#ifndef DMAP_LEAF32_MIN_BLOCKS
-#define DMAP_LEAF32_MIN_BLOCKS 1
-#endif
-template <bool ST, typename R, typename H, typename Fp>
-__global__ void __launch_bounds__(128, DMAP_LEAF32_MIN_BLOCKS)
-    wave_leaf32(const TriDev32 *__restrict__ tris32, const TriDev *__restrict__ tris64,
-                const AssetDev *__restrict__ assets, const R *__restrict__ rays, dmapk::QueryOpts opt,
-                H *__restrict__ hits, int64_t *__restrict__ stats, RayState *__restrict__ states,
-                const LeafJob *__restrict__ q_leaf, int round, int *__restrict__ q_out, unsigned long long *ctr,
-                int *__restrict__ rerun)
-{
-    using namespace d64;
-    constexpr int kDepth = 5; // subdivision_depth
-    enum : int { NEED = 0, SETUP = 1, SEARCH = 2, DONE = 3 };
-    const int lane = threadIdx.x & 31;
-    const unsigned long long count = *round_ctr(ctr, round, 1);
-    unsigned long long *fetch = round_ctr(ctr, round, 2);
-    int phase = NEED;
-    unsigned long long item = 0;
-    int ray = 0, tri = 0, n_leaves = 0, q = 0, li = 0, lj = 0, sp = 0;
-    bool first = false, answered = false;
-    double t_min = 0.0, t_max = 0.0;
-    v3 O = V3(0.0, 0.0, 0.0), D = O;
-    l32::Leaf32 L;
-    l32::Ent32 stack[4 * kDepth + 4];
-    int64_t subs = 0, iters = 0;
-
-    for (;;) {
-        unsigned need = __ballot_sync(FULL, phase == NEED);
-        if (need) {
-            int leader = __ffs(need) - 1;
-            unsigned long long base = 0;
-            if (lane == leader)
-                base = atomicAdd(fetch, (unsigned long long)__popc(need));
-            base = __shfl_sync(FULL, base, leader);
-            if (phase == NEED) {
-                item = base + (unsigned long long)__popc(need & ((1u << lane) - 1u));
-                if (item >= count) {
-                    phase = DONE;
-                } else {
-                    const LeafJob &J = q_leaf[item];
-                    ray = J.ray;
-                    tri = J.tri;
-                    n_leaves = J.n;
-                    q = 0;
-                    if (n_leaves == 0) {
-                        unsigned long long slot = atomicAdd(round_ctr(ctr, round, 3), 1ull);
-                        q_out[slot] = ray;
-                    } else {
-                        double o[3], d[3];
-                        load_ray(rays, ray, o, d, t_min, t_max);
-                        if (tris64[tri].inst) {
-                            double oo[3], od[3];
-                            dmapdev::object_ray(opt.inst_xf + dmapdev::kInstDoubles * (tris64[tri].inst - 1), o, d,
-                                                oo, od);
-                            for (int a = 0; a < 3; ++a) {
-                                o[a] = oo[a];
-                                d[a] = od[a];
-                            }
-                        }
-                        O = V3(o[0], o[1], o[2]);
-                        D = V3(d[0], d[1], d[2]);
-                        t_max = states[ray].t_max;
-                        answered = false;
-                        subs = iters = 0;
-                        phase = SETUP;
-                    }
-                }
-            }
-        }
-        if (__all_sync(FULL, phase == DONE))
-            break;
-        const TriDev &T = tris64[tri];
-        const AssetDev &g = assets[T.asset];
-        if (phase == SETUP) {
-            li = q_leaf[item].i[q];
-            lj = q_leaf[item].j[q];
-            l32::leaf_setup32(T, g, O, D, li, lj, L);
-            sp = 0;
-            stack[sp++] = {0.5f, 0.5f, -INFINITY, 0};
-            first = true;
-            phase = SEARCH;
-        }
-        bool expand = false, newton = false;
-        l32::Ent32 e = {0.0f, 0.0f, 0.0f, 0};
-        if (phase == SEARCH) {
-            while (sp > 0) {
-                e = stack[--sp];
-                if (first || (double)e.t_lo < t_max) {
-                    first = false;
-                    newton = e.depth == kDepth;
-                    expand = !newton;
-                    break;
-                }
-            }
-            if (!expand && !newton) {
-                if (++q < n_leaves && !answered) {
-                    phase = SETUP;
-                } else {
-                    if (ST) {
-                        stats[DMAP_ST_N * (int64_t)ray + DMAP_ST_SUB] += subs;
-                        stats[DMAP_ST_N * (int64_t)ray + DMAP_ST_NEWTON] += iters;
-                    }
-                    if (!answered) {
-                        unsigned long long slot = atomicAdd(round_ctr(ctr, round, 3), 1ull);
-                        q_out[slot] = ray;
-                    }
-                    phase = NEED;
-                }
-            }
-        }
-        __syncwarp();
-        if (expand) {
-            const TriDev32 &T32 = tris32[tri];
-            float r = __int_as_float((125 - e.depth) << 23); // half of the entry's rho = 0.5 * 2^-depth
-            l32::Ent32 ch[4];
-            int n = 0;
-#pragma unroll 1
-            for (int k = 0; k < 4; ++k) {
-                float ca = e.a + ((k & 1) ? r : -r), cb = e.b + ((k & 2) ? r : -r), tl;
-                ++subs;
-                if (l32::sub_square_bound32(T32, L, ca, cb, r, t_min, t_max, tl))
-                    ch[n++] = {ca, cb, tl, e.depth + 1};
-            }
-            for (int p = 1; p < n; ++p)
-                for (int k = p; k > 0 && ch[k].t_lo < ch[k - 1].t_lo; --k) {
-                    l32::Ent32 x = ch[k];
-                    ch[k] = ch[k - 1];
-                    ch[k - 1] = x;
-                }
-            for (int k = n - 1; k >= 0; --k)
-                stack[sp++] = ch[k];
-        }
-        __syncwarp();
-        if (newton) {
-            l32::Root32 root;
-            hit64 h;
-            int fl = 0;
-            if (l32::newton32(T, L, e.a, e.b, root, iters) &&
-                l32::accept_root(T, g, L.lo_s, L.lo_t, L.w, L.Q3, L.inv_dlen, O, D, t_min, t_max, li, lj, root,
-                                 opt.polish_cond, h, fl, iters)) {
-                t_max = h.t;
-                RayState &s = states[ray];
-                s.t_max = h.t;
-                s.best_tri = tri;
-                s.flags |= kFoundInTri | kShrunk;
-                s.nah = s.lah = 0;
-                if (tris64[tri].inst)
-                    dmapdev::world_normal(opt.inst_xf + dmapdev::kInstDoubles * (tris64[tri].inst - 1), h.ng);
-                store_hit<H, Fp>(hits, ray, true, h, tri, fl | ((s.flags & kCapped) ? DMAP_HIT_CAPPED : 0));
-                check_crossing(opt, tris64[tri], tri, h, ray, s.flags, ctr, rerun);
-                if (opt.mode == 1) {
-                    answered = true;
-                    sp = 0;
-                }
-            }
-        }
-        __syncwarp();
-    }
+    report();
 }
 
 int sm_count()

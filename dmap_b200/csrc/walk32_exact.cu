@@ -57,61 +57,37 @@ cudaError_t walk_drain(const Args &a, const int *q_in, int round, cudaStream_t s
     return cudaGetLastError();
 }
 
-template <typename R>
 cudaError_t filter(const Args &a, int round, cudaStream_t stream)
 {
-    wave_filter<R><<<sm_count() * 4, 128, 0, stream>>>(a.t64, a.assets, static_cast<const R *>(a.rays), a.opt,
-                                                       static_cast<RayState *>(a.states),
-                                                       static_cast<LeafJob *>(a.leaves), round, a.counters);
+    wave_filter<<<a.filter_grid, 128, 0, stream>>>(a.t64, a.assets, a.rays, a.opt, static_cast<RayState *>(a.states),
+                                                   static_cast<LeafJob *>(a.leaves), round, a.counters);
     return cudaGetLastError();
 }
 
-template <typename R, typename H, typename Fp>
-cudaError_t leaf64(const Args &a, int round, int *q_out, cudaStream_t stream)
+cudaError_t leaves(const Args &a, int round, int *q_out, cudaStream_t stream)
 {
-    const int lgrid = sm_count() * 4;
-    const R *rr = static_cast<const R *>(a.rays);
-    H *hh = static_cast<H *>(a.hits);
     RayState *states = static_cast<RayState *>(a.states);
-    LeafJob *leaves = static_cast<LeafJob *>(a.leaves);
-    if (a.stats)
-        wave_leaf<true, R, H, Fp><<<lgrid, 128, 0, stream>>>(a.t64, a.assets, rr, a.opt, hh, a.stats, states, leaves,
-                                                            round, q_out, a.counters, a.rerun);
+    const LeafJob *jobs = static_cast<const LeafJob *>(a.leaves);
+#define DMAP_LEAVES(ST_, P_)                                                                                        \
+    wave_leaf<ST_, P_><<<a.leaf_grid, kLeafThreads, 0, stream>>>(a.t32, a.t64, a.assets, a.rays, a.opt, a.hits,     \
+                                                                 ST_ ? a.stats : nullptr, states, jobs, round,      \
+                                                                 q_out, a.counters, a.rerun)
+    if (a.opt.leaf_precision == 1) // the FP32 certified leaf
+        a.stats ? DMAP_LEAVES(true, lq::P32) : DMAP_LEAVES(false, lq::P32);
     else
-        wave_leaf<false, R, H, Fp><<<lgrid, 128, 0, stream>>>(a.t64, a.assets, rr, a.opt, hh, nullptr, states,
-                                                             leaves, round, q_out, a.counters, a.rerun);
-    return cudaGetLastError();
-}
-
-template <typename R, typename H, typename Fp>
-cudaError_t leaf32(const Args &a, int round, int *q_out, cudaStream_t stream)
-{
-    const int lgrid = sm_count() * 4;
-    const R *rr = static_cast<const R *>(a.rays);
-    H *hh = static_cast<H *>(a.hits);
-    RayState *states = static_cast<RayState *>(a.states);
-    LeafJob *leaves = static_cast<LeafJob *>(a.leaves);
-    if (a.stats)
-        wave_leaf32<true, R, H, Fp><<<lgrid, 128, 0, stream>>>(a.t32, a.t64, a.assets, rr, a.opt, hh, a.stats, states,
-                                                              leaves, round, q_out, a.counters, a.rerun);
-    else
-        wave_leaf32<false, R, H, Fp><<<lgrid, 128, 0, stream>>>(a.t32, a.t64, a.assets, rr, a.opt, hh, nullptr,
-                                                               states, leaves, round, q_out, a.counters, a.rerun);
+        a.stats ? DMAP_LEAVES(true, lq::P64) : DMAP_LEAVES(false, lq::P64);
+#undef DMAP_LEAVES
     return cudaGetLastError();
 }
 
 #define DMAP_W32_EXACT(R, H, Fp)                                                                                    \
     template cudaError_t simple<R, H, Fp>(const Args &, cudaStream_t);                                              \
-    template cudaError_t simple_rerun<R, H, Fp>(const Args &, cudaStream_t);                                        \
-    template cudaError_t leaf64<R, H, Fp>(const Args &, int, int *, cudaStream_t);                                  \
-    template cudaError_t leaf32<R, H, Fp>(const Args &, int, int *, cudaStream_t);
+    template cudaError_t simple_rerun<R, H, Fp>(const Args &, cudaStream_t);
 DMAP_W32_EXACT(float, dmapdev::Hit32, float)
 DMAP_W32_EXACT(float, dmapdev::Hit64, double)
 DMAP_W32_EXACT(double, dmapdev::Hit32, float)
 DMAP_W32_EXACT(double, dmapdev::Hit64, double)
 #undef DMAP_W32_EXACT
-template cudaError_t filter<float>(const Args &, int, cudaStream_t);
-template cudaError_t filter<double>(const Args &, int, cudaStream_t);
 
 } // namespace w32
 } // namespace dmapk

@@ -29,7 +29,7 @@ struct Args
     void *leaves;                 // wavefront: the leaf jobs
     unsigned long long *counters; // wavefront: kWaveCounters
     int *rerun;                   // wavefront, filtered scene: rays the filter's schedule answers again
-    int grid;                     // wavefront: walk CTAs
+    int grid, filter_grid, leaf_grid; // wavefront: CTAs of the walk, the cell filter and the leaves
 };
 
 // walk32_exact.cu
@@ -39,12 +39,8 @@ cudaError_t simple(const Args &a, cudaStream_t stream);
 template <typename R, typename H, typename Fp>
 cudaError_t simple_rerun(const Args &a, cudaStream_t stream);
 cudaError_t walk_drain(const Args &a, const int *q_in, int round, cudaStream_t stream);
-template <typename R>
 cudaError_t filter(const Args &a, int round, cudaStream_t stream);
-template <typename R, typename H, typename Fp>
-cudaError_t leaf64(const Args &a, int round, int *q_out, cudaStream_t stream);
-template <typename R, typename H, typename Fp>
-cudaError_t leaf32(const Args &a, int round, int *q_out, cudaStream_t stream);
+cudaError_t leaves(const Args &a, int round, int *q_out, cudaStream_t stream);
 
 // walk32.cu
 cudaError_t walk_round(const Args &a, const int *q_in, int round, cudaStream_t stream);

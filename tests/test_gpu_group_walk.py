@@ -76,3 +76,22 @@ def test_deep_charts(ctx, oracle, tiles, rounds):
     assert dev.triangle_info(0)[0] == levels[tiles]
     for order in ("nearest", "index"):
         assert _equal(cpu, dev, rays, order, rounds) > 100
+
+
+@pytest.mark.parametrize("leaf", ["f32", "f64"])
+@pytest.mark.parametrize("n", [1, 3, 8, 31, 500, 6000])
+def test_leaf_rounds_agree(ctx, oracle, n, leaf):
+    """The leaf kernel's batches (set up eight jobs at a time, searched by
+    quads, records made in batches) against the last walk's inline leaves
+    (rounds 0): the same records however the leaves are split, and the
+    occlusion answers of the closest-hit query."""
+    sc = helpers.small_sphere(32)
+    cpu, dev = py_oracle.CpuScene(oracle, sc), dm.Scene.from_synthetic(ctx, sc)
+    rays = helpers.aimed_rays(cpu, n, seed=n)[0]
+    base = dev.intersect(rays, dm.TraversalOptions(rounds=0, leaf_precision=leaf), np.float64)
+    for rounds in (1, 2, 3):
+        h = dev.intersect(rays, dm.TraversalOptions(rounds=rounds, leaf_precision=leaf), np.float64)
+        assert np.array_equal(h.tobytes(), base.tobytes())
+    for rounds in (0, 1, 2):
+        o = dev.intersect(rays, dm.TraversalOptions(rounds=rounds, leaf_precision=leaf, mode="occluded"), np.float64)
+        assert np.array_equal(o["tri"] >= 0, base["tri"] >= 0)
