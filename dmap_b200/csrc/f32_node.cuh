@@ -233,6 +233,27 @@ __device__ __forceinline__ void box_axis(float a0, float au, float av, float cx,
     hi = __fadd_ru(hi, gw);
 }
 
+// a / b as a product with the hardware's reciprocal (rcp.approx: within 1
+// ulp), rounded up / down past its error, for |b| between 1e-30 and 1e30,
+// whose reciprocal is a normal float.
+__device__ __forceinline__ bool quot_ok(float b) { return fabsf(b) > 1e-30f && fabsf(b) < 1e30f; }
+__device__ __forceinline__ float approx_rcp(float b)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+    return r;
+}
+__device__ __forceinline__ float quot_up(float a, float b)
+{
+    const float q = a * approx_rcp(b);
+    return __fmaf_ru(fabsf(q), 4.76837158203125e-07f, q);
+}
+__device__ __forceinline__ float quot_dn(float a, float b)
+{
+    const float q = a * approx_rcp(b);
+    return __fmaf_rd(-fabsf(q), 4.76837158203125e-07f, q);
+}
+
 // The node test of one cell (node_bounds.cpp:83-211): the box, and at levels
 // <= slab_max_level the slab, both enclosing their double counterparts.
 __device__ __forceinline__ bool node_test32(const Walk32 &T, const float *pyr32, const Ray32 &r, int level, int i,
@@ -290,19 +311,26 @@ __device__ __forceinline__ bool node_test32(const Walk32 &T, const float *pyr32,
     float span = c1 - c0;
     Iv F0 = iv_add(iv_add(iv_add(iv_scale(az, A), iv_scale(ax, B)), iv_scale(ay, C)), D);
     Iv F1 = iv_add(iv_add(iv_scale(r.dz, A), iv_scale(r.dx, B)), iv_scale(r.dy, C));
+    // the quotients of the interval test as products with a reciprocal within
+    // 2^-23, widened by 2^-21; a divisor out of its range bounds nothing
     float s0 = 0.0f, s1 = span;
-    if (F1.lo > 0.0f)
-        s1 = fminf(s1, __fdiv_ru(__fsub_ru(R, F0.lo), F1.lo));
-    else if (F1.lo < 0.0f)
-        s0 = fmaxf(s0, __fdiv_rd(__fsub_ru(R, F0.lo), F1.lo));
-    else if (F0.lo > R)
+    const float ql = __fsub_ru(R, F0.lo), qh = __fsub_rd(-R, F0.hi);
+    if (quot_ok(F1.lo)) {
+        if (F1.lo > 0.0f)
+            s1 = fminf(s1, quot_up(ql, F1.lo));
+        else
+            s0 = fmaxf(s0, quot_dn(ql, F1.lo));
+    } else if (F1.lo == 0.0f && F0.lo > R) {
         return false;
-    if (F1.hi > 0.0f)
-        s0 = fmaxf(s0, __fdiv_rd(__fsub_rd(-R, F0.hi), F1.hi));
-    else if (F1.hi < 0.0f)
-        s1 = fminf(s1, __fdiv_ru(__fsub_rd(-R, F0.hi), F1.hi));
-    else if (F0.hi < -R)
+    }
+    if (quot_ok(F1.hi)) {
+        if (F1.hi > 0.0f)
+            s0 = fmaxf(s0, quot_dn(qh, F1.hi));
+        else
+            s1 = fminf(s1, quot_up(qh, F1.hi));
+    } else if (F1.hi == 0.0f && F0.hi < -R) {
         return false;
+    }
     if (s0 > s1 + tol32(fabsf(c0) + span))
         return false;
     if (bound == 1)

@@ -152,10 +152,11 @@ struct leafent { double a, b, t_lo; int depth; };
 __device__ inline void leaf_setup(const TriDev &T, const AssetDev &g, v3 o, v3 d, int64_t i, int64_t j, leafbound &L)
 {
     L.place(g, i, j);
-    L.h00 = grid_h(g, L.lo.x, L.lo.y);
-    L.h10 = grid_h(g, L.lo.x + L.w, L.lo.y);
-    L.h01 = grid_h(g, L.lo.x, L.lo.y + L.w);
-    L.h11 = grid_h(g, L.lo.x + L.w, L.lo.y + L.w);
+    double hc[4];
+#pragma unroll 1
+    for (int q = 0; q < 4; ++q)
+        hc[q] = grid_h(g, (q & 1) ? L.lo.x + L.w : L.lo.x, (q & 2) ? L.lo.y + L.w : L.lo.y);
+    L.h00 = hc[0], L.h10 = hc[1], L.h01 = hc[2], L.h11 = hc[3];
     v2 c = add2(L.lo, V2(0.5 * L.w, 0.5 * L.w));
     double hw = 0.5 * L.w;
     L.N_hat = AF3(add3(add3(L3(T.m0), mul3(c.x, L3(T.Mu))), mul3(c.y, L3(T.Mv))), mul3(hw, L3(T.Mu)),
@@ -165,6 +166,26 @@ __device__ inline void leaf_setup(const TriDev &T, const AssetDev &g, v3 o, v3 d
     L.d_len = norm3(d);
     L.dn = div3(d, L.d_len);
     plane_basis(L.dn, L.d1, L.d2);
+}
+
+// Out-of-line copies, shared by every caller of a translation unit: the
+// wavefront's kernels are bound by instruction fetch where their loops hold
+// several inlined copies of these.
+static __device__ __noinline__ void leaf_setup_shared(const TriDev &T, const AssetDev &g, v3 o, v3 d, int64_t i,
+                                                      int64_t j, leafbound &L)
+{
+    leaf_setup(T, g, o, d, i, j, L);
+}
+static __device__ __noinline__ bool newton_from_shared(const TriDev &T, const AssetDev &g, v3 o, v3 d, double t_min,
+                                                       double t_max, int64_t i, int64_t j, v2 guess, hit64 &hit,
+                                                       int64_t &iters)
+{
+    return newton_from(T, g, o, d, t_min, t_max, i, j, guess, hit, iters);
+}
+static __device__ __noinline__ void root_record_shared(const TriDev &T, const AssetDev &g, double t, v2 st, int64_t i,
+                                                       int64_t j, hit64 &hit)
+{
+    root_record(T, g, t, st, i, j, hit);
 }
 
 // intersect_newton + search_leaf (:239-264, :292-323) with an explicit

@@ -77,8 +77,11 @@ __device__ inline void leaf_setup32(const TriDev &T, const AssetDev &g, v3 o, v3
 {
     L.place(g, i, j);
     const double w = L.w, los = L.lo_s, lot = L.lo_t;
-    double h00 = grid_h(g, los, lot), h10 = grid_h(g, los + w, lot);
-    double h01 = grid_h(g, los, lot + w), h11 = grid_h(g, los + w, lot + w);
+    double hc[4]; // one copy of the lookup's code: the leaf kernels wait on instruction fetch
+#pragma unroll 1
+    for (int q = 0; q < 4; ++q)
+        hc[q] = grid_h(g, (q & 1) ? los + w : los, (q & 2) ? lot + w : lot);
+    const double h00 = hc[0], h10 = hc[1], h01 = hc[2], h11 = hc[3];
     double hm = 0.25 * ((h00 + h10) + (h01 + h11));
     L.hmid = (float)hm;
     L.d00 = (float)(h00 - hm);
@@ -134,6 +137,12 @@ __device__ inline void leaf_setup32(const TriDev &T, const AssetDev &g, v3 o, v3
                    (fabs(h00 - hm) + fabs(h10 - h00) + fabs(h01 - h00) + fabs(h11 - h10 - h01 + h00));
     double tol = fmax(T.residual_tol, 2.384185791015625e-07 * scale); // 2^-22
     L.tol2 = (float)(tol * tol);
+}
+
+static __device__ __noinline__ void leaf_setup32_shared(const TriDev &T, const AssetDev &g, v3 o, v3 d, int64_t i,
+                                                        int64_t j, Leaf32 &L)
+{
+    leaf_setup32(T, g, o, d, i, j, L);
 }
 
 // sub_square_bound (:266-290) over the sub-square (a, b) +- rho of the texel,
@@ -289,7 +298,7 @@ __device__ __forceinline__ bool judge_root(const TriDev &T, const AssetDev &g, c
         int64_t it = 0;
         v3 o, d;
         ray(o, d);
-        bool ok = newton_from(T, g, o, d, t_min, INFINITY, i, j, st, h, it);
+        bool ok = newton_from_shared(T, g, o, d, t_min, INFINITY, i, j, st, h, it);
         iters += it;
         if (ok) {
             if (h.t >= t_max)
@@ -318,7 +327,7 @@ static __device__ __noinline__ bool accept_root(const TriDev &T, const AssetDev 
     if (!judge_root(T, g, L, ray, t_min, t_max, i, j, R, polish_cond, t, st, fl, iters))
         return false;
     flags = fl;
-    root_record(T, g, t, st, i, j, hit);
+    root_record_shared(T, g, t, st, i, j, hit);
     return true;
 }
 
@@ -332,7 +341,7 @@ __device__ inline bool intersect_newton32(const TriDev &T, const TriDev32 &T32, 
 {
     constexpr int kDepth = 5; // subdivision_depth
     Leaf32 L;
-    leaf_setup32(T, g, o, d, i, j, L);
+    leaf_setup32_shared(T, g, o, d, i, j, L);
     bool found = false;
     int64_t subs = 0, iters = 0;
     Ent32 stack[4 * kDepth + 4];

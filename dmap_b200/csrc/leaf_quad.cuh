@@ -43,7 +43,7 @@ struct P32
     struct Ent { float a, b, t_lo; int depth; };
     static __device__ __forceinline__ void setup(const TriDev &T, const AssetDev &g, v3 o, v3 d, int i, int j, Bound &L)
     {
-        l32::leaf_setup32(T, g, o, d, i, j, L);
+        l32::leaf_setup32_shared(T, g, o, d, i, j, L);
     }
     // a stored setup's leaf, for the cell and the ray it was made for
     template <class Ray>
@@ -80,7 +80,7 @@ struct P64
     struct Ent { double t_lo; float a, b; int depth; }; // a, b: multiples of 2^-6, exact
     static __device__ __forceinline__ void setup(const TriDev &T, const AssetDev &g, v3 o, v3 d, int i, int j, Bound &L)
     {
-        d64::leaf_setup(T, g, o, d, i, j, L);
+        d64::leaf_setup_shared(T, g, o, d, i, j, L);
     }
     template <class Ray>
     static __device__ __forceinline__ void place(const AssetDev &g, const Ray &ray, int i, int j, Bound &L)

@@ -61,13 +61,12 @@ using dmapdev::AssetDev;
 using dmapdev::TriDev;
 using dmapdev::TriDev32;
 
-// Resident 128-thread CTAs per SM the walk is compiled for (register budget:
-// 65536 / (128 x blocks) per thread). The walk rounds over the per-ray
-// candidate mask (scenes of up to 256 triangles) take 4 (112 registers, no
-// spills); over the triangle tree, whose candidate buffer lives in local
-// memory either way, 5.
+// Resident 128-thread CTAs per SM the walk rounds are compiled for (register
+// budget: 65536 / (128 x blocks) per thread; 96 registers at 5). 2.80M rays on
+// the sphere of 96 x 2048^2 maps, walk rounds at 4 / 5 / 6: 18.3 / 16.3 / 16.2
+// ms; 20,011 rays on 512^2 maps 0.43 / 0.45 / 0.49.
 #ifndef DMAP_WALK_MIN_BLOCKS
-#define DMAP_WALK_MIN_BLOCKS 4
+#define DMAP_WALK_MIN_BLOCKS 5
 #endif
 #ifndef DMAP_WALK_TREE_MIN_BLOCKS
 #define DMAP_WALK_TREE_MIN_BLOCKS 5
@@ -85,22 +84,20 @@ constexpr unsigned FULL = 0xffffffffu;
 // ray and the reference's double ray (A (o - q0), A d in its own operation
 // order): the rounding to float, at most 2^-24 of each coordinate (2^-22
 // taken), plus the difference of two double evaluations of the transform,
-// a few units of 2^-53 of the sums of the terms' magnitudes (2^-40 taken).
+// a few units of 2^-53 of the sums of the terms' magnitudes (2^-40 taken of
+// the row's magnitude sum times the largest component). tangent_row: axis a.
 __device__ __forceinline__ void tangent_row(const TriDev32 &T, int a, const double *o, const double *d, float t_far,
                                             float &ro, float &rd, float &e)
 {
     const double A0 = T.A[a][0], A1 = T.A[a][1], A2 = T.A[a][2];
-    double u0 = o[0] - T.q0[0], u1 = o[1] - T.q0[1], u2 = o[2] - T.q0[2];
-    double x = A0 * u0;
-    x = __fma_rn(A1, u1, x);
-    x = __fma_rn(A2, u2, x);
-    double y = __fma_rn(A2, d[2], __fma_rn(A1, d[1], A0 * d[0]));
-    double mx = fabs(A0 * u0) + fabs(A1 * u1) + fabs(A2 * u2);
-    double my = fabs(A0 * d[0]) + fabs(A1 * d[1]) + fabs(A2 * d[2]);
-    ro = (float)x;
-    rd = (float)y;
-    float sum = ru_add(__double2float_ru(mx), ru_mul(t_far, __double2float_ru(my)));
-    e = ru_add(ru_mul(0x1p-22f, ru_add(fabsf(ro), ru_mul(t_far, fabsf(rd)))), ru_mul(0x1p-40f, sum));
+    const double u0 = o[0] - T.q0[0], u1 = o[1] - T.q0[1], u2 = o[2] - T.q0[2];
+    const double d0 = d[0], d1 = d[1], d2 = d[2];
+    ro = (float)__fma_rn(A2, u2, __fma_rn(A1, u1, A0 * u0));
+    rd = (float)__fma_rn(A2, d2, __fma_rn(A1, d1, A0 * d0));
+    const float um = fmaxf(fmaxf(fabsf((float)u0), fabsf((float)u1)), fabsf((float)u2));
+    const float dm = fmaxf(fmaxf(fabsf((float)d0), fabsf((float)d1)), fabsf((float)d2));
+    const float sum = ru_mul(__double2float_ru(fabs(A0) + fabs(A1) + fabs(A2)), ru_fma(t_far, dm, um));
+    e = ru_fma(0x1p-22f, ru_fma(t_far, fabsf(rd), fabsf(ro)), ru_mul(0x1.1p-40f, sum));
 }
 
 __device__ __forceinline__ void tangent_ray(const TriDev32 &T, const double *o, const double *d, float t_far,
@@ -115,6 +112,23 @@ __device__ __forceinline__ void tangent_ray(const TriDev32 &T, const double *o, 
 }
 
 __device__ __forceinline__ float far_bound(float t1) { return ru_add(ru_mul(t1, 1.0f + 4.0f * G), G); }
+
+// Position of the k-th set bit (k from 0) of m, or -1.
+__device__ __forceinline__ int nth_bit(unsigned m, int k)
+{
+#pragma unroll 1
+    for (; k > 0; --k)
+        m &= m - 1u;
+    return __ffs((int)m) - 1;
+}
+// m without its k lowest set bits.
+__device__ __forceinline__ unsigned drop_bits(unsigned m, int k)
+{
+#pragma unroll 1
+    for (; k > 0; --k)
+        m &= m - 1u;
+    return m;
+}
 
 // ---- simple schedule: one thread per ray ----------------------------------
 
@@ -457,6 +471,18 @@ __device__ __forceinline__ unsigned long long *round_ctr(unsigned long long *c, 
     return c + 4 * round + k;
 }
 
+// Ray k as triangle T meets it: in the object space of an instanced one
+// (instance.cuh). One copy of its code for the leaf kernels.
+__device__ __noinline__ void leaf_ray(const void *rays, int ray_dtype, int64_t k, const double *inst_xf, int inst,
+                                      d64::v3 &O, d64::v3 &D, double &t_min, double &t_max)
+{
+    double o[3], d[3], oo[3], od[3];
+    load_ray(rays, ray_dtype, k, o, d, t_min, t_max);
+    dmapdev::ray_for(inst_xf, inst, o, d, oo, od);
+    O = d64::V3(oo[0], oo[1], oo[2]);
+    D = d64::V3(od[0], od[1], od[2]);
+}
+
 // A leaf cell the last walk reached, by the four lanes of its ray's quad: the
 // cell's FP64 node test, then the certified leaf in the query's precision.
 // A nearer root is stored as the ray's hit; returns the ray's t_max.
@@ -470,18 +496,9 @@ __device__ __noinline__ double quad_leaf(const TriDev32 &T32, const TriDev &T, c
     const lq::Quad Q = {0xfu << (lane & 28), lane & 28, lane & 3};
     const AssetDev &g = assets[T.asset];
     typename P::Ent *stack = reinterpret_cast<typename P::Ent *>(stack_mem);
-    double o[3], d[3], t_min, t_ray;
-    load_ray(rays, opt.ray_dtype, ray, o, d, t_min, t_ray);
-    if (T.inst) {
-        // an instanced triangle meets the ray in its object space (instance.cuh)
-        double oo[3], od[3];
-        dmapdev::object_ray(opt.inst_xf + dmapdev::kInstDoubles * (T.inst - 1), o, d, oo, od);
-        for (int a = 0; a < 3; ++a) {
-            o[a] = oo[a];
-            d[a] = od[a];
-        }
-    }
-    const d64::v3 O = d64::V3(o[0], o[1], o[2]), D = d64::V3(d[0], d[1], d[2]);
+    double t_min, t_ray;
+    d64::v3 O, D;
+    leaf_ray(rays, opt.ray_dtype, ray, opt.inst_xf, T.inst, O, D, t_min, t_ray);
     if (!d64::leaf_cell_admitted(T, g, O, D, t_min, t_max, i, j, opt))
         return t_max;
     typename P::Bound L;
@@ -514,7 +531,7 @@ __device__ __noinline__ double quad_leaf(const TriDev32 &T32, const TriDev &T, c
     } while (lq::pop<P>(stack, sp, t_max, e));
     if (mine == t_max && t_max < t_start) {
         d64::hit64 h;
-        d64::root_record(T, g, best.t, best.st, i, j, h);
+        d64::root_record_shared(T, g, best.t, best.st, i, j, h);
         if (T.inst)
             dmapdev::world_normal(opt.inst_xf + dmapdev::kInstDoubles * (T.inst - 1), h.ng);
         store_hit(hits, opt.hit_dtype, ray, true, h, tri, best.flags | ((flags & kCapped) ? DMAP_HIT_CAPPED : 0));
@@ -531,6 +548,42 @@ __device__ __noinline__ double quad_leaf(const TriDev32 &T32, const TriDev &T, c
     return t_max;
 }
 
+// A round's rays per warp are fetched in at least this many parts.
+#ifndef DMAP_RAY_SPLIT
+#define DMAP_RAY_SPLIT 4ull
+#endif
+
+// A ray in work or fetched ahead, as its picks read it.
+struct RaySlot
+{
+    double o[3], d[3], inv[3], t_min, t_max; // inv: d64::ray_inverse
+    float of[3], df[3], invf[3];
+    int ray;
+};
+
+// The slabs of a box against a ray (d32::box_range), out of line: one copy of
+// its code serves every place of the walk that tests a box. Component c of
+// the box is box[c * stride]. pass() false: the ray misses it; t1 is the exit
+// bound either way.
+struct Span
+{
+    float t0, t1;
+    bool ok;
+    __device__ __forceinline__ bool pass() const { return ok; }
+};
+__device__ __noinline__ Span box_span(const float *box, int stride, const RaySlot &S, float t0, float t1)
+{
+    float lo[3], hi[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        lo[c] = box[c * stride];
+        hi[c] = box[(3 + c) * stride];
+    }
+    Span r = {t0, t1, false};
+    r.ok = box_range(lo, hi, S.of, S.df, S.invf, r.t0, r.t1);
+    return r;
+}
+
 // Four lanes walk one ray (a quad; eight rays per warp), so that the four
 // cells of a sibling group are tested together, one per lane. A lane per ray
 // ran one node test per step with 19.6 of 32 lanes in it, the others being in
@@ -538,7 +591,14 @@ __device__ __noinline__ double quad_leaf(const TriDev32 &T32, const TriDev &T, c
 // time of small batches and of every launch's tail. Walk rounds and last walk
 // before and after: 64 rays on a quad 212 -> 63 us, 20,011 rays on the sphere
 // of 96 x 512^2 maps 2.80 -> 0.69 ms, 2.80M rays on 96 x 2048^2 34.1 -> 27.2
-// ms. Per quad and step: take
+// ms.
+//
+// The loop's code is kept small: at 53 KB (the box test in four places, the
+// park in four, the ray transform and the ray's load in two each) 2.7 of 8.6
+// cycles per issued instruction were instruction fetch, at 84 KB 7.2 of 13.
+// Each now stands in one place (40 KB), and rays are fetched ahead, a lane
+// per ray, into shared memory: the walk rounds above take 16.4 ms from 22.5.
+// Per quad and step: take
 // the next cell of the open groups (its lowest bit), descend into it by
 // testing its four children, or collect it when it is a leaf.
 //
@@ -590,15 +650,11 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
         }
         __syncthreads();
     }
+    // the rays in work and those the warp has fetched ahead
+    constexpr int kRaySlots = INLINE_LEAF ? 16 : 32, kRayBatch = kRaySlots - 8; // per warp, eight in work
+    __shared__ RaySlot s_ray[4][kRaySlots];
     // the last walk: the leaf search's stacks, per quad
     __shared__ double s_stack[INLINE_LEAF ? 32 : 1][INLINE_LEAF ? lq::kStack * sizeof(lq::P64::Ent) / 8 : 1];
-    auto box32 = [&](int t, float *lo, float *hi) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            lo[c] = s_box32[c * kStaged + t];
-            hi[c] = s_box32[(3 + c) * kStaged + t];
-        }
-    };
     // items of this round: every ray in round 0, else the resume queue
     unsigned long long count = round == 0 ? (unsigned long long)n : *round_ctr(ctr, round - 1, 3);
     if (round == 0 && opt.n_dev && (unsigned long long)*opt.n_dev < count)
@@ -608,6 +664,13 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
     // its warps, so that fewer of them share a warp
     const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
     int phase = (unsigned long long)(lane >> 2) * warps < count ? NEED : DONE;
+    // rays fetched at once: up to kRayBatch, fewer in a round of few rays per warp
+    const int batch = (int)max(1ull, min((unsigned long long)kRayBatch, count / (DMAP_RAY_SPLIT * warps)));
+    bool more = count > 0ull; // rays may be left in the queue
+    unsigned ready = 0u;      // slots with a ray no quad has taken
+    const int wi = threadIdx.x >> 5;
+    RaySlot *const slots = s_ray[wi];
+    int slot = 0; // the quad's ray
     int ray = 0;
     double t_max = 0.0;
     float tmin_f = 0.0f, tmax_f = 0.0f;
@@ -695,84 +758,109 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
     };
 
     for (;;) {
-        // 1. quads without work take the next items, one atomic per warp
-        const unsigned need = __ballot_sync(FULL, phase == NEED) & 0x11111111u;
+        // 1. quads without work take a ray that is ready; when none is, the
+        // warp fetches the next ones of the round, a lane per ray
         bool fresh = false;
-        float of[3], df[3], invf[3]; // the ray in float, while it is fetched or picks
-        if (need) {
-            const int leader = __ffs(need) - 1;
-            unsigned long long base = 0;
-            if (lane == leader)
-                base = atomicAdd(fetch, (unsigned long long)__popc(need));
-            base = __shfl_sync(FULL, base, leader);
-            if (phase == NEED) {
-                unsigned long long item = base + (unsigned long long)__popc(need & ((1u << lead) - 1u));
-                if (item >= count) {
-                    phase = DONE;
-                } else {
-                    ray = round == 0 ? (int)item : q_in[item];
-                    double o[3], d[3], t_min;
-                    load_ray(rays, opt.ray_dtype, ray, o, d, t_min, t_max);
-                    nbuf.n = -1;
+        bool enter = false; // the quad's lanes need the ray in triangle tri's frame
+        unsigned need;
+        while ((need = __ballot_sync(FULL, phase == NEED) & 0x11111111u) != 0u) {
+            if (!ready) {
+                if (!more) {
+                    if (phase == NEED)
+                        phase = DONE;
+                    break;
+                }
+                unsigned long long base = 0;
+                if (lane == 0)
+                    base = atomicAdd(fetch, (unsigned long long)batch);
+                base = __shfl_sync(FULL, base, 0);
+                more = base + batch < count;
+                const unsigned taken = __reduce_or_sync(FULL, phase == TOP || phase == WALK ? 1u << slot : 0u);
+                const bool get = lane < batch && base + lane < count;
+                const int to = get ? nth_bit(~taken, lane) : 0;
+                if (get) {
+                    RaySlot &S = slots[to];
+                    const int k = round == 0 ? (int)(base + lane) : q_in[base + lane];
+                    double o[3], d[3], t0, t1;
+                    load_ray(rays, opt.ray_dtype, k, o, d, t0, t1);
 #pragma unroll
                     for (int a = 0; a < 3; ++a) {
-                        of[a] = (float)o[a];
-                        df[a] = (float)d[a];
-                        invf[a] = df[a] != 0.0f ? __frcp_rn(df[a]) : 0.0f;
+                        S.o[a] = o[a];
+                        S.d[a] = d[a];
+                        S.of[a] = (float)o[a];
+                        S.df[a] = (float)d[a];
                     }
-                    tmin_f = __double2float_rd(t_min);
-                    if (ST)
-                        for (int q = 0; q < DMAP_ST_N; ++q)
-                            stl[q] = 0;
-                    if (round == 0) {
-                        tri = 0;
-                        ckey = -INFINITY;
-                        cidx = -1;
-                        best_tri = -1;
-                        flags = 0;
-                        mask = 0ull;
-                        tmax_f = __double2float_ru(t_max);
-                        fresh = true;
-                        phase = TOP;
+#pragma unroll 1
+                    for (int a = 0; a < 3; ++a) {
+                        S.inv[a] = S.d[a] != 0.0 ? 1.0 / S.d[a] : 0.0; // d64::ray_inverse
+                        S.invf[a] = S.df[a] != 0.0f ? __frcp_rn(S.df[a]) : 0.0f;
+                    }
+                    S.t_min = t0;
+                    S.t_max = t1;
+                    S.ray = k;
+                }
+                __syncwarp();
+                ready = __reduce_or_sync(FULL, get ? 1u << to : 0u);
+                continue;
+            }
+            const int k = __popc(need & ((1u << lead) - 1u)), want = __popc(need);
+            if (phase == NEED && k < __popc(ready)) {
+                slot = nth_bit(ready, k);
+                const RaySlot &S = slots[slot];
+                ray = S.ray;
+                tmin_f = __double2float_rd(S.t_min);
+                nbuf.n = -1;
+                if (ST)
+                    for (int q = 0; q < DMAP_ST_N; ++q)
+                        stl[q] = 0;
+                if (round == 0) {
+                    t_max = S.t_max;
+                    tri = 0;
+                    ckey = -INFINITY;
+                    cidx = -1;
+                    best_tri = -1;
+                    flags = 0;
+                    mask = 0ull;
+                    tmax_f = __double2float_ru(t_max);
+                    fresh = true;
+                    phase = TOP;
+                } else {
+                    const RayState &s = states[ray];
+                    t_max = s.t_max;
+                    tri = s.tri;
+                    best_tri = s.best_tri;
+                    flags = s.flags;
+                    cur = {s.cl, s.ci, s.cj};
+                    todo.lo = s.todo[0];
+                    dom.lo = s.dom[0];
+                    if (DEEP) {
+                        todo.hi = s.todo[1];
+                        dom.hi = s.dom[1];
+                    }
+                    if (ST) {
+                        nah = s.nah;
+                        lah = s.lah;
+                    }
+                    if (TREE) {
+                        ckey = s.ckey;
+                        cidx = s.cidx;
+                        if (sub == 0)
+                            nbuf = s.buf;
                     } else {
-                        const RayState &s = states[ray];
-                        t_max = s.t_max;
-                        tri = s.tri;
-                        best_tri = s.best_tri;
-                        flags = s.flags;
-                        cur = {s.cl, s.ci, s.cj};
-                        todo.lo = s.todo[0];
-                        dom.lo = s.dom[0];
-                        if (DEEP) {
-                            todo.hi = s.todo[1];
-                            dom.hi = s.dom[1];
-                        }
-                        if (ST) {
-                            nah = s.nah;
-                            lah = s.lah;
-                        }
-                        if (TREE) {
-                            ckey = s.ckey;
-                            cidx = s.cidx;
-                            if (sub == 0)
-                                nbuf = s.buf;
-                        } else {
-                            mask = s.mask[sub];
-                        }
-                        // back into the walk just after the leaves (displaced_intersector.cpp:229)
-                        tmax_f = __double2float_ru(t_max);
-                        const TriDev32 &T = tris32[tri];
-                        float t1 = tmax_f;
-                        object_box(T, of, df, invf, tmin_f, t1);
-                        enter_frame(T, o, d, far_bound(fmaxf(t1, tmin_f)));
-                        stale = (flags & kShrunk) ? ~0u : 0u;
-                        flags &= ~kShrunk;
-                        guard = 0;
-                        nl = 0;
-                        phase = WALK;
+                        mask = s.mask[sub];
                     }
+                    // back into the walk just after the leaves (displaced_intersector.cpp:229)
+                    tmax_f = __double2float_ru(t_max);
+                    enter = true;
+                    stale = (flags & kShrunk) ? ~0u : 0u;
+                    flags &= ~kShrunk;
+                    guard = 0;
+                    nl = 0;
+                    phase = WALK;
                 }
             }
+            ready = drop_bits(ready, want);
+            __syncwarp();
         }
         // round 0: the warp finds the fresh rays' candidate triangles
         // together, 32 boxes per ballot; byte q of a ballot is the triangles
@@ -782,23 +870,12 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
             while (left) {
                 const int src = __ffs(left) - 1;
                 left &= left - 1;
-                float so[3], sd[3], sv[3];
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    so[a] = __shfl_sync(FULL, of[a], src);
-                    sd[a] = __shfl_sync(FULL, df[a], src);
-                    sv[a] = __shfl_sync(FULL, invf[a], src);
-                }
+                const RaySlot &S = slots[__shfl_sync(FULL, slot, src)];
                 const float s_tmin = __shfl_sync(FULL, tmin_f, src), s_tmax = __shfl_sync(FULL, tmax_f, src);
 #pragma unroll 1
                 for (int w = 0; w < ((n_tri + 31) >> 5); ++w) {
                     const int t = 32 * w + 4 * (lane & 7) + (lane >> 3);
-                    float t1 = s_tmax, lo[3], hi[3];
-                    bool pass = t < n_tri;
-                    if (pass) {
-                        box32(t, lo, hi);
-                        pass = box_pass(lo, hi, so, sd, sv, s_tmin, t1);
-                    }
+                    const bool pass = t < n_tri && box_span(s_box32 + t, kStaged, S, s_tmin, s_tmax).pass();
                     const unsigned bits = __ballot_sync(FULL, pass);
                     if (lead == src)
                         mask |= (unsigned long long)((bits >> (8 * sub)) & 255u) << (8 * w);
@@ -809,30 +886,15 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
             break;
 
         // 2. the next triangle whose object box the ray meets (intersect_flat's loop)
+        float t1 = tmax_f; // the exit bound of the triangle's box
         bool test = false, roots = false, again = false; // a group to test: the roots; one tested before
         if (phase == TOP) {
             const unsigned quad = 0xfu << lead;
-            double o[3], d[3], t_min, t_ray;
-            load_ray(rays, opt.ray_dtype, ray, o, d, t_min, t_ray);
-            if (!fresh) {
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    of[a] = (float)o[a];
-                    df[a] = (float)d[a];
-                    invf[a] = df[a] != 0.0f ? __frcp_rn(df[a]) : 0.0f;
-                }
-            }
-            float t1 = 0.0f;
+            const RaySlot &S = slots[slot];
+            const double *o = S.o, *d = S.d, *inv = S.inv;
+            const float *of = S.of, *df = S.df, *invf = S.invf;
+            const double t_min = S.t_min;
             int bt = -1;
-            double inv[3];
-            if (NEAR) {
-                // 1 / d in double, an axis per lane
-                const double da = sub == 0 ? d[0] : sub == 1 ? d[1] : d[2];
-                const double ia = da != 0.0 ? 1.0 / da : 0.0;
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
-                    inv[a] = __shfl_sync(quad, ia, lead + a);
-            }
             if (TREE) {
                 if (sub == 0) {
                     bool err = false;
@@ -863,38 +925,40 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                 // bit is cleared too, so every bit left is past it.
                 double bk = 0.0;
                 unsigned long long m = mask;
+#pragma unroll 1
                 while (m) {
                     const int b = __ffsll((long long)m) - 1;
                     m &= m - 1ull;
                     const int t = 4 * b + sub;
-                    float e = tmin_f, tt = tmax_f, lo[3], hi[3];
-                    box32(t, lo, hi);
-                    if (!box_range(lo, hi, of, df, invf, e, tt)) {
+                    const Span x = box_span(s_box32 + t, kStaged, S, tmin_f, tmax_f);
+                    if (!x.pass()) {
                         mask &= ~(1ull << b);
                         continue;
                     }
                     if (!NEAR) {
                         bt = t;
-                        t1 = tt;
+                        t1 = x.t1;
                         break;
                     }
-                    if (bt >= 0 && (double)e > bk)
-                        continue; // its key (at least e) is past the best
-                    double dlo[3], dhi[3];
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        dlo[c] = s_box64[c * kStaged + t];
-                        dhi[c] = s_box64[(3 + c) * kStaged + t];
-                    }
-                    const double key = d64::entry_key(dlo, dhi, o, d, inv, t_min);
+                    if (bt >= 0 && (double)x.t0 > bk)
+                        continue; // its key (at least its entry) is past the best
+                    // d64::entry_key
+                    double key = t_min;
+#pragma unroll 1
+                    for (int a = 0; a < 3; ++a)
+                        if (d[a] != 0.0) {
+                            const double oa = o[a], ia = inv[a];
+                            key = d64::dmax(key, d64::dmin((s_box64[a * kStaged + t] - oa) * ia,
+                                                           (s_box64[(3 + a) * kStaged + t] - oa) * ia));
+                        }
                     if (!d64::before_best(key, t, bk, bt))
                         continue;
                     bk = key;
                     bt = t;
-                    t1 = tt;
+                    t1 = x.t1;
                 }
                 __syncwarp(quad);
-#pragma unroll
+#pragma unroll 1
                 for (int x = 1; x < 4; x <<= 1) {
                     const int ot = __shfl_xor_sync(quad, bt, x);
                     const float o1 = __shfl_xor_sync(quad, t1, x);
@@ -925,7 +989,7 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                 phase = NEED;
             } else {
                 tri = bt;
-                enter_frame(tris32[tri], o, d, far_bound(t1));
+                enter = true;
                 todo = {0ull, 0ull};
                 dom = {0ull, 0ull};
                 stale = 0u;
@@ -937,6 +1001,15 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                 phase = WALK;
                 test = roots = true;
             }
+        }
+        if (enter) {
+            const TriDev32 &T = tris32[tri];
+            if (!test) {
+                // a resumed ray: the exit bound with the current t_max
+                const Span x = box_span(T.box_lo, 1, slots[slot], tmin_f, tmax_f);
+                t1 = fmaxf(x.t1, tmin_f);
+            }
+            enter_frame(T, slots[slot].o, slots[slot].d, far_bound(t1));
         }
         __syncwarp();
 
@@ -958,7 +1031,8 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                     test = false;
                 }
             }
-            while (!test && phase == WALK) {
+            bool parking = false;
+            while (!test && phase == WALK && !parking) {
                 if (!todo.any()) {
                     // the end of the triangle's walk
                     if (ST) {
@@ -969,7 +1043,7 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                     dom = {0ull, 0ull};
                     if (!INLINE_LEAF && nl > 0) {
                         // the collected leaves decide this triangle's t_max before the next one
-                        park();
+                        parking = true;
                     } else {
                         if (ST && (flags & kFoundInTri)) {
                             stl[DMAP_ST_NAH] += nah;
@@ -1009,7 +1083,7 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                                 ++nah;
                             }
                         }
-                        park();
+                        parking = true;
                         break;
                     }
                     since += n_in;
@@ -1020,7 +1094,7 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                 }
                 dom.clear_upto(p);
                 if (l > 0 && nl > 0 && since > DMAP_STALE_CAP) {
-                    park(); // the cell is taken (and its group tested) again after the resume
+                    parking = true; // the cell is taken (and its group tested) again after the resume
                     break;
                 }
                 todo.clear_bit(p);
@@ -1051,8 +1125,10 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                 if (nl == 0)
                     since = 1;
                 if (++nl == DMAP_COLLECT || since > DMAP_STALE_CAP)
-                    park();
+                    parking = true;
             }
+            if (!INLINE_LEAF && parking)
+                park();
         }
         __syncwarp();
 
@@ -1112,43 +1188,6 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
     }
 }
 
-// The leaf cells of a round's jobs through the reference's own node test in
-// double (node_bounds.cpp:83-211 at level 0, the node computed from the
-// grid), a lane per cell: the FP32 walk, widened by its roundings, reaches
-// more leaf cells than the FP64 walk, and a cell the FP64 walk rejects has no
-// leaf there. The ray's t_max is the one it parked with; earlier leaves of
-// the same job can only shrink it, so a cell kept here may still be rejected
-// by the FP64 walk at that point, and its search then finds nothing the
-// reference would not. Kept apart from the leaf kernel so that kernel's code
-// stays small.
-__global__ void __launch_bounds__(128)
-    wave_filter(const TriDev *__restrict__ tris64, const AssetDev *__restrict__ assets, const void *__restrict__ rays,
-                dmapk::QueryOpts opt, const RayState *__restrict__ states, LeafJob *__restrict__ q_leaf, int round,
-                const unsigned long long *ctr)
-{
-    const unsigned long long count = 4ull * *round_ctr(const_cast<unsigned long long *>(ctr), round, 1);
-    const int lead = threadIdx.x & 28, sub = threadIdx.x & 3;
-    for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; k < count;
-         k += (unsigned long long)gridDim.x * blockDim.x) {
-        LeafJob &job = q_leaf[k >> 2];
-        bool admitted = false;
-        if (sub < job.n) {
-            double o[3], d[3], oo[3], od[3], t_min, t_max;
-            load_ray(rays, opt.ray_dtype, job.ray, o, d, t_min, t_max);
-            t_max = states[job.ray].t_max;
-            const TriDev &T = tris64[job.tri];
-            dmapdev::ray_for(opt.inst_xf, T.inst, o, d, oo, od);
-            admitted = d64::leaf_cell_admitted(T, assets[T.asset], d64::V3(oo[0], oo[1], oo[2]),
-                                               d64::V3(od[0], od[1], od[2]), t_min, t_max, job.i[sub], job.j[sub], opt);
-        }
-        const unsigned quad = 0xfu << lead;
-        __syncwarp(quad);
-        const unsigned keep = __ballot_sync(quad, admitted);
-        if (sub == 0)
-            job.keep = (int)((keep >> lead) & 15u);
-    }
-}
-
 // The parked leaves of a round, a quad per job: the cells the filter kept are
 // searched in walk order, all four lanes together (leaf_quad.cuh), one entry
 // per step, quads at the same kind of step side by side. A ray whose walk has
@@ -1199,7 +1238,7 @@ __global__ void __launch_bounds__(kLeafThreads,
     constexpr int kRecs = 32;  // leaf setups per warp
     constexpr int kReps = 16;  // hit records per warp still to be made
     __shared__ Bound s_rec[kLeafThreads / 32][kRecs];
-    struct Slot { int ray, tri, keep, i[kCollect], j[kCollect]; unsigned char rec[kCollect]; };
+    struct Slot { double t_min; int ray, tri, keep, i[kCollect], j[kCollect]; unsigned char rec[kCollect]; };
     __shared__ Slot s_job[kLeafThreads / 32][kSlots];
     __shared__ Ent s_stack[kLeafThreads / 4][lq::kStack];
     // the root each quad's job holds, and the roots of finished jobs whose
@@ -1231,18 +1270,8 @@ __global__ void __launch_bounds__(kLeafThreads,
 
     // the job's ray, in its triangle's space
     auto ray_of = [&](v3 &O, v3 &D) {
-        double o[3], d[3], t0, t1;
-        load_ray(rays, opt.ray_dtype, ray, o, d, t0, t1);
-        const int inst = tris64[tri].inst;
-        if (inst) {
-            double oo[3], od[3];
-            dmapdev::object_ray(opt.inst_xf + dmapdev::kInstDoubles * (inst - 1), o, d, oo, od);
-            O = V3(oo[0], oo[1], oo[2]);
-            D = V3(od[0], od[1], od[2]);
-        } else {
-            O = V3(o[0], o[1], o[2]);
-            D = V3(d[0], d[1], d[2]);
-        }
+        double t0, t1;
+        leaf_ray(rays, opt.ray_dtype, ray, opt.inst_xf, tris64[tri].inst, O, D, t0, t1);
     };
     // the records of the roots found, a lane per root
     auto report = [&]() {
@@ -1251,7 +1280,7 @@ __global__ void __launch_bounds__(kLeafThreads,
             const Rep &r = s_rep[wi][lane];
             const TriDev &T = tris64[r.tri];
             hit64 h;
-            root_record(T, assets[T.asset], r.t, V2(r.s, r.v), r.i, r.j, h);
+            root_record_shared(T, assets[T.asset], r.t, V2(r.s, r.v), r.i, r.j, h);
             if (T.inst)
                 dmapdev::world_normal(opt.inst_xf + dmapdev::kInstDoubles * (T.inst - 1), h.ng);
             RayState &s = states[r.ray];
@@ -1270,21 +1299,19 @@ __global__ void __launch_bounds__(kLeafThreads,
             if (ready) {
                 const int k = __popc(need & ((1u << Q.lead) - 1u)), have = __popc(ready), want = __popc(need);
                 if (phase == NEED && k < have) {
-                    slot = (int)__fns(ready, 0, k + 1);
+                    slot = nth_bit(ready, k);
                     const Slot &J = s_job[wi][slot];
                     ray = J.ray;
                     tri = J.tri;
                     keep = (unsigned)J.keep;
-                    double o[3], d[3];
-                    load_ray(rays, opt.ray_dtype, ray, o, d, t_min, t_max);
+                    t_min = J.t_min;
                     t_max = states[ray].t_max;
                     sp = 0;
                     subs = iters = 0;
                     answered = found = false;
                     phase = SEARCH;
                 }
-                for (int q = 0; q < want; ++q)
-                    ready &= ready - 1u;
+                ready = drop_bits(ready, want);
                 __syncwarp();
                 continue;
             }
@@ -1324,7 +1351,7 @@ __global__ void __launch_bounds__(kLeafThreads,
             next += __popc(took);
             // the slots no quad's job is in
             const unsigned taken = __reduce_or_sync(FULL, phase == SEARCH || phase == NEWTON ? 1u << slot : 0u);
-            const int to = (int)__fns(~taken, 0, (lane >> 2) + 1);
+            const int to = nth_bit(~taken, (lane >> 2));
             unsigned mine = 0u;
             if (fits) {
                 Slot &S = s_job[wi][to];
@@ -1338,14 +1365,15 @@ __global__ void __launch_bounds__(kLeafThreads,
                 S.i[Q.sub] = li;
                 S.j[Q.sub] = lj;
                 if ((cells >> Q.sub) & 1u) {
-                    const int at = (int)__fns(~recs, 0, __popc(kept & ((1u << lane) - 1u)) + 1);
+                    const int at = nth_bit(~recs, __popc(kept & ((1u << lane) - 1u)));
                     S.rec[Q.sub] = (unsigned char)at;
                     mine = 1u << at;
-                    double o[3], d[3], oo[3], od[3], t0, t1;
-                    load_ray(rays, opt.ray_dtype, jr, o, d, t0, t1);
+                    double t0, t1;
+                    v3 O, D;
                     const TriDev &T = tris64[jt];
-                    dmapdev::ray_for(opt.inst_xf, T.inst, o, d, oo, od);
-                    P::setup(T, assets[T.asset], V3(oo[0], oo[1], oo[2]), V3(od[0], od[1], od[2]), li, lj, s_rec[wi][at]);
+                    leaf_ray(rays, opt.ray_dtype, jr, opt.inst_xf, T.inst, O, D, t0, t1);
+                    S.t_min = t0; // the same from every lane
+                    P::setup(T, assets[T.asset], O, D, li, lj, s_rec[wi][at]);
                 }
             }
             __syncwarp();

@@ -6,6 +6,46 @@
 // round it finishes in).
 #include "walk32.cuh"
 
+namespace
+{
+// The leaf cells of a round's jobs through the reference's own node test in
+// double (node_bounds.cpp:83-211 at level 0, the node computed from the
+// grid), a lane per cell: the FP32 walk, widened by its roundings, reaches
+// more leaf cells than the FP64 walk, and a cell the FP64 walk rejects has no
+// leaf there. The ray's t_max is the one it parked with; earlier leaves of
+// the same job can only shrink it, so a cell kept here may still be rejected
+// by the FP64 walk at that point, and its search then finds nothing the
+// reference would not. Kept apart from the leaf kernel so that kernel's code
+// stays small.
+__global__ void __launch_bounds__(128)
+    wave_filter(const TriDev *__restrict__ tris64, const AssetDev *__restrict__ assets, const void *__restrict__ rays,
+                dmapk::QueryOpts opt, const RayState *__restrict__ states, LeafJob *__restrict__ q_leaf, int round,
+                const unsigned long long *ctr)
+{
+    const unsigned long long count = 4ull * *round_ctr(const_cast<unsigned long long *>(ctr), round, 1);
+    const int lead = threadIdx.x & 28, sub = threadIdx.x & 3;
+    for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; k < count;
+         k += (unsigned long long)gridDim.x * blockDim.x) {
+        LeafJob &job = q_leaf[k >> 2];
+        bool admitted = false;
+        if (sub < job.n) {
+            double t_min, t_max;
+            d64::v3 O, D;
+            const TriDev &T = tris64[job.tri];
+            leaf_ray(rays, opt.ray_dtype, job.ray, opt.inst_xf, T.inst, O, D, t_min, t_max);
+            t_max = states[job.ray].t_max;
+            admitted = d64::leaf_cell_admitted(T, assets[T.asset], O, D, t_min, t_max, job.i[sub], job.j[sub], opt);
+        }
+        const unsigned quad = 0xfu << lead;
+        __syncwarp(quad);
+        const unsigned keep = __ballot_sync(quad, admitted);
+        if (sub == 0)
+            job.keep = (int)((keep >> lead) & 15u);
+    }
+}
+
+} // namespace
+
 namespace dmapk
 {
 namespace w32
