@@ -22,7 +22,7 @@ cudaError_t walk_round(const Args &a, const int *q_in, int round, cudaStream_t s
     RayState *states = static_cast<RayState *>(a.states);
     LeafJob *leaves = static_cast<LeafJob *>(a.leaves);
 #define DMAP_ROUND(ST_, TR_, NR_, DP_)                                                                              \
-    wave_walk<ST_, false, TR_, NR_, DP_><<<a.grid, 128, 0, stream>>>(                                     \
+    wave_walk<ST_, false, TR_, NR_, DP_><<<a.grid, 128, entry_bytes(a.n_tri), stream>>>(                                     \
         a.t32, a.t64, a.n_tri, a.assets, a.rays, a.n, a.opt, a.hits, ST_ ? a.stats : nullptr, states, q_in, round, leaves,  \
         a.counters, a.status, a.rerun)
 #define DMAP_ROUND_DEEP(ST_, TR_, NR_)                                                                              \

@@ -548,11 +548,6 @@ __device__ __noinline__ double quad_leaf(const TriDev32 &T32, const TriDev &T, c
     return t_max;
 }
 
-// A round's rays per warp are fetched in at least this many parts.
-#ifndef DMAP_RAY_SPLIT
-#define DMAP_RAY_SPLIT 4ull
-#endif
-
 // A ray in work or fetched ahead, as its picks read it.
 struct RaySlot
 {
@@ -561,17 +556,24 @@ struct RaySlot
     int ray;
 };
 
-// The slabs of a box against a ray (d32::box_range), out of line: one copy of
-// its code serves every place of the walk that tests a box. Component c of
-// the box is box[c * stride]. pass() false: the ray misses it; t1 is the exit
-// bound either way.
+// An empty slab range beyond the FP32 tolerance (box_range's test; with wide
+// 2 and t_lo the range's start, node_range's).
+__device__ __forceinline__ bool misses(float t0, float t1, float wide, float t_lo)
+{
+    return t0 > t1 + wide * tol32(fmaxf(fmaxf(fabsf(t0), fabsf(t1)), fabsf(t_lo)));
+}
+
+// The slabs of a box against a ray (d32::box_range, or with wide 2 and t_lo
+// node_range), out of line: one copy of its code serves every place of the
+// walk that tests a box. Component c of the box is box[c * stride]. Not ok:
+// the ray misses it; t1 is the exit bound either way.
 struct Span
 {
     float t0, t1;
     bool ok;
-    __device__ __forceinline__ bool pass() const { return ok; }
 };
-__device__ __noinline__ Span box_span(const float *box, int stride, const RaySlot &S, float t0, float t1)
+__device__ __noinline__ Span box_span(const float *box, int stride, const RaySlot &S, float t0, float t1,
+                                      float wide = 1.0f, float t_lo = 0.0f)
 {
     float lo[3], hi[3];
 #pragma unroll
@@ -580,8 +582,21 @@ __device__ __noinline__ Span box_span(const float *box, int stride, const RaySlo
         hi[c] = box[(3 + c) * stride];
     }
     Span r = {t0, t1, false};
-    r.ok = box_range(lo, hi, S.of, S.df, S.invf, r.t0, r.t1);
+    r.ok = box_slabs(lo, hi, S.of, S.df, S.invf, r.t0, r.t1) && !misses(r.t0, r.t1, wide, t_lo);
     return r;
+}
+
+// d64::entry_key of a box (lo, then hi), out of line.
+__device__ __noinline__ double box_key(const double *lo, const RaySlot &S)
+{
+    double key = S.t_min;
+#pragma unroll 1
+    for (int a = 0; a < 3; ++a)
+        if (S.d[a] != 0.0) {
+            const double o = S.o[a], inv = S.inv[a];
+            key = d64::dmax(key, d64::dmin((lo[a] - o) * inv, (lo[3 + a] - o) * inv));
+        }
+    return key;
 }
 
 // Four lanes walk one ray (a quad; eight rays per warp), so that the four
@@ -613,6 +628,25 @@ __device__ __noinline__ Span box_span(const float *box, int stride, const RaySlo
 // which runs the few rays left with their leaves inline, for
 // DMAP_DRAIN_MIN_BLOCKS, so that the leaf it calls is not squeezed into the
 // rounds' register budget.
+// In a round that keeps the quads busy (32 rays and more per warp), the warp
+// makes its picks when DMAP_PICK_QUADS of its quads (TREE:
+// DMAP_TREE_PICK_QUADS) need one, or none has a group to test: a pick costs
+// about as much as a group's test and served 1.9 quads. Over the tree, whose
+// refills cost several times that, fetches wait too. 2.80M rays on 96 x
+// 2048^2 maps, walk rounds at 1 / 2 / 3 / 4: 15.9 / 15.3 / 15.0 / 15.1 ms;
+// 12,288 triangles 6.2 / 5.4 / 5.2 / 5.1. In the last walk a leaf waits for
+// DMAP_DRAIN_QUADS: 1 / 2 / 3 / 4 / 6: 3.6 / 3.0 / 2.8 / 2.6 / 2.6 ms, and in
+// index order with the FP64 leaf (100,003 rays) 3.5 / 3.0 / 2.7 / 2.6 / 2.3.
+// Small rounds, where a ray's own chain sets the time, wait for nothing.
+#ifndef DMAP_PICK_QUADS
+#define DMAP_PICK_QUADS 3
+#endif
+#ifndef DMAP_TREE_PICK_QUADS
+#define DMAP_TREE_PICK_QUADS 4
+#endif
+#ifndef DMAP_DRAIN_QUADS
+#define DMAP_DRAIN_QUADS 6
+#endif
 #ifndef DMAP_DRAIN_MIN_BLOCKS
 #define DMAP_DRAIN_MIN_BLOCKS 2
 #endif
@@ -625,7 +659,7 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
               const int *__restrict__ q_in, int round, LeafJob *__restrict__ q_leaf, unsigned long long *ctr,
               unsigned *status, int *__restrict__ rerun)
 {
-    enum : int { NEED = 0, TOP = 1, WALK = 2, DONE = 3 };
+    enum : int { NEED = 0, TOP = 1, WALK = 2, DONE = 3, LEAF = 4 }; // LEAF: the last walk, at a leaf cell
     const int lane = threadIdx.x & 31, sub = lane & 3, lead = lane & 28;
     // the candidates: scenes of up to 256 triangles take a mask of one bit
     // per triangle whose box the ray meets (built by the warp at the ray's
@@ -634,24 +668,34 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
     // the mask only for up to 256 triangles, so its loops are never compiled
     // into the kernels of larger scenes
     const d32::BvhView bvh = {opt.bvh_nodes, opt.bvh_tri, opt.bvh_range, opt.bvh_n_nodes};
-    // scenes of up to 256 triangles: their object boxes in shared memory
-    // (outward FP32 for the box tests, FP64 for the nearest order's keys),
-    // which every candidate test of the CTA reads; component c of triangle t
-    // at c * kStaged + t
+    // scenes of up to 256 triangles: their outward FP32 boxes in shared
+    // memory, component c of triangle t at c * kStaged + t
     constexpr int kStaged = TREE ? 1 : 32 * kMaskWords;
     __shared__ float s_box32[6 * kStaged];
-    __shared__ double s_box64[(NEAR ? 6 : 1) * kStaged];
     if (!TREE) {
         for (int k = threadIdx.x; k < 6 * n_tri; k += blockDim.x) {
             const int t = k / 6, c = k - 6 * t;
             s_box32[c * kStaged + t] = c < 3 ? tris32[t].box_lo[c] : tris32[t].box_hi[c - 3];
-            if (NEAR)
-                s_box64[c * kStaged + t] = c < 3 ? tris64[t].box_lo[c] : tris64[t].box_hi[c - 3];
         }
         __syncthreads();
     }
+    // boxes around runs of 8 triangles, for the candidates' first test
+    constexpr int kRuns = TREE ? 1 : 32;
+    __shared__ float s_run[6 * kRuns];
+    if (!TREE) {
+        for (int k = threadIdx.x; k < 6 * kRuns; k += blockDim.x) {
+            const int c = k >> 5, first = 8 * (k & 31);
+            float v = c < 3 ? INFINITY : -INFINITY;
+            for (int t = first; t < first + 8 && t < n_tri; ++t)
+                v = c < 3 ? fminf(v, s_box32[c * kStaged + t]) : fmaxf(v, s_box32[c * kStaged + t]);
+            s_run[k] = v;
+        }
+        __syncthreads();
+    }
+    // the box entries of a lane's candidates: of mask bit b at b * 128 + thread
+    extern __shared__ float s_entry[];
     // the rays in work and those the warp has fetched ahead
-    constexpr int kRaySlots = INLINE_LEAF ? 16 : 32, kRayBatch = kRaySlots - 8; // per warp, eight in work
+    constexpr int kRaySlots = 16, kRayBatch = 8; // per warp: eight in work, eight ahead
     __shared__ RaySlot s_ray[4][kRaySlots];
     // the last walk: the leaf search's stacks, per quad
     __shared__ double s_stack[INLINE_LEAF ? 32 : 1][INLINE_LEAF ? lq::kStack * sizeof(lq::P64::Ent) / 8 : 1];
@@ -664,8 +708,14 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
     // its warps, so that fewer of them share a warp
     const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
     int phase = (unsigned long long)(lane >> 2) * warps < count ? NEED : DONE;
-    // rays fetched at once: up to kRayBatch, fewer in a round of few rays per warp
-    const int batch = (int)max(1ull, min((unsigned long long)kRayBatch, count / (DMAP_RAY_SPLIT * warps)));
+    // rays fetched at once: a fill of the warp's quads while at least two
+    // fills per warp are to come, else a quarter of the warp's share, so that
+    // no warp is left with several long rays (20,011 rays, 7 per warp: the
+    // walk rounds take 0.43 ms, with half of the share at once 0.45; 65,536
+    // rays on one quad, 22 per warp: 156 us with a fill, 171 with a quarter)
+    const int batch = count >= 2ull * kRayBatch * warps ? kRayBatch : (int)max(1ull, count / (4ull * warps));
+    const bool full = !INLINE_LEAF && count >= 32ull * warps;
+    const int pick_quads = full ? (TREE ? DMAP_TREE_PICK_QUADS : DMAP_PICK_QUADS) : 1;
     bool more = count > 0ull; // rays may be left in the queue
     unsigned ready = 0u;      // slots with a ray no quad has taken
     const int wi = threadIdx.x >> 5;
@@ -688,7 +738,8 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
     Cell32 cur = {0, 0, 0};
     CellBits<DEEP> todo = {0ull, 0ull}, dom = {0ull, 0ull}; // cells that passed; cells in the domain, not yet gone past
     unsigned stale = 0u;                                   // levels whose group must be tested again
-    unsigned long long mask = 0ull;
+    unsigned long long mask = 0ull; // the lane's candidates
+    bool entries = false;           // their box entries are in s_entry
     int64_t stl[DMAP_ST_N];
     int nl = 0, li = 0, lj = 0; // collected leaves, the lane's own
     int since = 0;              // node tests since the first collected leaf
@@ -764,6 +815,8 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
         bool enter = false; // the quad's lanes need the ray in triangle tri's frame
         unsigned need;
         while ((need = __ballot_sync(FULL, phase == NEED) & 0x11111111u) != 0u) {
+            if (TREE && __popc(need) < pick_quads && __any_sync(FULL, phase == WALK || phase == TOP || phase == LEAF))
+                break;
             if (!ready) {
                 if (!more) {
                     if (phase == NEED)
@@ -775,7 +828,7 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                     base = atomicAdd(fetch, (unsigned long long)batch);
                 base = __shfl_sync(FULL, base, 0);
                 more = base + batch < count;
-                const unsigned taken = __reduce_or_sync(FULL, phase == TOP || phase == WALK ? 1u << slot : 0u);
+                const unsigned taken = __reduce_or_sync(FULL, phase != NEED && phase != DONE ? 1u << slot : 0u);
                 const bool get = lane < batch && base + lane < count;
                 const int to = get ? nth_bit(~taken, lane) : 0;
                 if (get) {
@@ -810,6 +863,7 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                 ray = S.ray;
                 tmin_f = __double2float_rd(S.t_min);
                 nbuf.n = -1;
+                entries = round == 0;
                 if (ST)
                     for (int q = 0; q < DMAP_ST_N; ++q)
                         stl[q] = 0;
@@ -863,8 +917,9 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
             __syncwarp();
         }
         // round 0: the warp finds the fresh rays' candidate triangles
-        // together, 32 boxes per ballot; byte q of a ballot is the triangles
-        // of lane q
+        // together: the runs the ray meets, then the boxes of four runs per
+        // ballot, lane 8 q + 2 i + k of a ballot triangle 4 k + q of its
+        // i-th run, so that byte q is the candidates of the quad's lane q
         if (!TREE) {
             unsigned left = __ballot_sync(FULL, fresh) & 0x11111111u;
             while (left) {
@@ -872,15 +927,26 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                 left &= left - 1;
                 const RaySlot &S = slots[__shfl_sync(FULL, slot, src)];
                 const float s_tmin = __shfl_sync(FULL, tmin_f, src), s_tmax = __shfl_sync(FULL, tmax_f, src);
+                unsigned runs = __ballot_sync(FULL, 8 * lane < n_tri && box_span(s_run + lane, kRuns, S, s_tmin, s_tmax,
+                                                                                 2.0f, s_tmin).ok);
 #pragma unroll 1
-                for (int w = 0; w < ((n_tri + 31) >> 5); ++w) {
-                    const int t = 32 * w + 4 * (lane & 7) + (lane >> 3);
-                    const bool pass = t < n_tri && box_span(s_box32 + t, kStaged, S, s_tmin, s_tmax).pass();
-                    const unsigned bits = __ballot_sync(FULL, pass);
-                    if (lead == src)
-                        mask |= (unsigned long long)((bits >> (8 * sub)) & 255u) << (8 * w);
+                while (runs) {
+                    const int run = nth_bit(runs, (lane & 7) >> 1), b = 2 * run + (lane & 1), t = 4 * b + (lane >> 3);
+                    bool ok = false;
+                    if (run >= 0 && t < n_tri) {
+                        const Span x = box_span(s_box32 + t, kStaged, S, s_tmin, s_tmax);
+                        ok = x.ok;
+                        if (ok)
+                            s_entry[b * 128 + (threadIdx.x & ~31) + src + (lane >> 3)] = x.t0;
+                    }
+                    const unsigned bits = __ballot_sync(FULL, ok);
+                    const unsigned own = lead == src ? (bits >> (8 * sub)) & 255u : 0u;
+#pragma unroll 1
+                    for (int i = 0; i < 8 && runs; i += 2, runs &= runs - 1u)
+                        mask |= (unsigned long long)((own >> i) & 3u) << (2 * (__ffs((int)runs) - 1));
                 }
             }
+            __syncwarp();
         }
         if (__all_sync(FULL, phase == DONE))
             break;
@@ -888,7 +954,9 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
         // 2. the next triangle whose object box the ray meets (intersect_flat's loop)
         float t1 = tmax_f; // the exit bound of the triangle's box
         bool test = false, roots = false, again = false; // a group to test: the roots; one tested before
-        if (phase == TOP) {
+        const unsigned top = __ballot_sync(FULL, phase == TOP) & 0x11111111u;
+        const bool pick = __popc(top) >= pick_quads || !__any_sync(FULL, phase == WALK);
+        if (phase == TOP && pick) {
             const unsigned quad = 0xfu << lead;
             const RaySlot &S = slots[slot];
             const double *o = S.o, *d = S.d, *inv = S.inv;
@@ -917,60 +985,98 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                 ckey = __shfl_sync(quad, ckey, lead);
                 cidx = __shfl_sync(quad, cidx, lead);
             } else {
-                // the best of each lane's candidates (nearest order: the
-                // smallest (key, index); index order: the smallest index),
-                // then of the quad's; each box is re-tested with the current
-                // t_max first, and a bit whose box no longer passes is
-                // cleared for good (t_max only shrinks). The taken triangle's
-                // bit is cleared too, so every bit left is past it.
-                double bk = 0.0;
-                unsigned long long m = mask;
+                // the entries of a resumed ray's candidates; those whose box
+                // no longer passes are dropped for good (t_max only shrinks)
+                if (!entries) {
 #pragma unroll 1
-                while (m) {
-                    const int b = __ffsll((long long)m) - 1;
-                    m &= m - 1ull;
-                    const int t = 4 * b + sub;
-                    const Span x = box_span(s_box32 + t, kStaged, S, tmin_f, tmax_f);
-                    if (!x.pass()) {
-                        mask &= ~(1ull << b);
-                        continue;
+                    for (unsigned long long m = mask; m; m &= m - 1ull) {
+                        const int b = __ffsll((long long)m) - 1;
+                        const Span x = box_span(s_box32 + 4 * b + sub, kStaged, S, tmin_f, tmax_f);
+                        s_entry[b * 128 + threadIdx.x] = x.t0;
+                        if (!x.ok)
+                            mask &= ~(1ull << b);
                     }
-                    if (!NEAR) {
-                        bt = t;
-                        t1 = x.t1;
-                        break;
-                    }
-                    if (bt >= 0 && (double)x.t0 > bk)
-                        continue; // its key (at least its entry) is past the best
-                    // d64::entry_key
-                    double key = t_min;
+                    entries = true;
+                }
 #pragma unroll 1
-                    for (int a = 0; a < 3; ++a)
-                        if (d[a] != 0.0) {
-                            const double oa = o[a], ia = inv[a];
-                            key = d64::dmax(key, d64::dmin((s_box64[a * kStaged + t] - oa) * ia,
-                                                           (s_box64[(3 + a) * kStaged + t] - oa) * ia));
+                for (;;) {
+                    // the quad's first candidate: in the nearest order the
+                    // smallest box entry, a lower bound of its key; in the
+                    // index order the smallest index
+                    float be = INFINITY;
+                    bt = -1;
+#pragma unroll 1
+                    for (unsigned long long m = mask; m; m &= m - 1ull) {
+                        const int b = __ffsll((long long)m) - 1;
+                        const float e = s_entry[b * 128 + threadIdx.x];
+                        if (e >= 0.0f && tmax_f >= 0.0f && e > tmax_f + tol32(fmaxf(e, tmax_f)))
+                            mask &= ~(1ull << b); // past t_max
+                        else if (bt < 0 || (NEAR && e < be)) {
+                            be = e;
+                            bt = 4 * b + sub;
                         }
-                    if (!d64::before_best(key, t, bk, bt))
-                        continue;
-                    bk = key;
-                    bt = t;
-                    t1 = x.t1;
-                }
-                __syncwarp(quad);
-#pragma unroll 1
-                for (int x = 1; x < 4; x <<= 1) {
-                    const int ot = __shfl_xor_sync(quad, bt, x);
-                    const float o1 = __shfl_xor_sync(quad, t1, x);
-                    const double ok = NEAR ? __shfl_xor_sync(quad, bk, x) : (double)ot;
-                    if (ot >= 0 && (NEAR ? d64::before_best(ok, ot, bk, bt) : (bt < 0 || ot < bt))) {
-                        bk = ok;
-                        bt = ot;
-                        t1 = o1;
                     }
+                    __syncwarp(quad);
+#pragma unroll 1
+                    for (int x = 1; x < 4; x <<= 1) {
+                        const int ot = __shfl_xor_sync(quad, bt, x);
+                        const float oe = __shfl_xor_sync(quad, be, x);
+                        if (ot >= 0 && (bt < 0 || (NEAR && oe < be) || ((!NEAR || oe == be) && ot < bt))) {
+                            be = oe;
+                            bt = ot;
+                        }
+                    }
+                    if (bt < 0)
+                        break;
+                    // it leaves the candidates, and is the next triangle if
+                    // its box passes with the current t_max
+                    const int first = bt;
+                    if ((bt & 3) == sub)
+                        mask &= ~(1ull << (bt >> 2));
+                    const Span x = box_span(s_box32 + bt, kStaged, S, tmin_f, tmax_f);
+                    t1 = x.t1;
+                    if (!x.ok)
+                        continue;
+                    if (!NEAR)
+                        break;
+                    // another candidate comes before it only if its entry is
+                    // not past this one's key: then their keys decide
+                    double bk = box_key(tris64[bt].box_lo, S);
+                    const double fk = bk;
+#pragma unroll 1
+                    for (unsigned long long m = mask; m; m &= m - 1ull) {
+                        const int b = __ffsll((long long)m) - 1, t = 4 * b + sub;
+                        if ((double)s_entry[b * 128 + threadIdx.x] > fk)
+                            continue;
+                        const Span y = box_span(s_box32 + t, kStaged, S, tmin_f, tmax_f);
+                        const double k = box_key(tris64[t].box_lo, S);
+                        if (y.ok && d64::before_best(k, t, bk, bt)) {
+                            bk = k;
+                            bt = t;
+                            t1 = y.t1;
+                        }
+                    }
+                    __syncwarp(quad);
+                    if (__any_sync(quad, bt != first)) {
+#pragma unroll 1
+                        for (int q = 1; q < 4; q <<= 1) {
+                            const int ot = __shfl_xor_sync(quad, bt, q);
+                            const float o1 = __shfl_xor_sync(quad, t1, q);
+                            const double ok = __shfl_xor_sync(quad, bk, q);
+                            if (d64::before_best(ok, ot, bk, bt)) {
+                                bk = ok;
+                                bt = ot;
+                                t1 = o1;
+                            }
+                        }
+                        // the taken one leaves, the first one stays
+                        if ((first & 3) == sub)
+                            mask |= 1ull << (first >> 2);
+                        if ((bt & 3) == sub)
+                            mask &= ~(1ull << (bt >> 2));
+                    }
+                    break;
                 }
-                if (bt >= 0 && (bt & 3) == sub)
-                    mask &= ~(1ull << (bt >> 2));
             }
             if (bt < 0) {
                 if (sub == 0) {
@@ -1017,7 +1123,6 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
         // cell's children are the group to test
         int tl = 0, pi = 0, pj = 0; // the group: its level, its parent cell
         unsigned cells = 15u;
-        bool leaf = false;
         if (phase == WALK) {
             const int root_level = tris32[tri].root_level;
             if (test) {
@@ -1114,7 +1219,7 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                     ++lah;
                 }
                 if (INLINE_LEAF) {
-                    leaf = true;
+                    phase = LEAF;
                     break;
                 }
                 // collect the leaf; park once DMAP_COLLECT are held
@@ -1133,8 +1238,13 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
         __syncwarp();
 
         if (INLINE_LEAF) {
-            // the last round: the few remaining rays finish here
-            if (leaf) {
+            // the last round: the few remaining rays finish here. A leaf
+            // waits until DMAP_DRAIN_QUADS quads of the warp have one, or no
+            // other has anything else to do.
+            const int wait = __popc(__ballot_sync(FULL, phase == LEAF) & 0x11111111u);
+            const bool others = __any_sync(FULL, phase == TOP || phase == WALK);
+            if (phase == LEAF && (wait >= DMAP_DRAIN_QUADS || !others)) {
+                phase = WALK;
                 const double t_old = t_max;
                 t_max = opt.leaf_precision == 1
                             ? quad_leaf<lq::P32, ST>(tris32[tri], tris64[tri], assets, rays, ray, tri, t_max, cur.i, cur.j,
@@ -1473,6 +1583,9 @@ __global__ void __launch_bounds__(kLeafThreads,
     }
     report();
 }
+
+// Dynamic shared memory of the walk: the candidates' box entries.
+size_t entry_bytes(int n_tri) { return n_tri > 32 * kMaskWords ? 0 : (size_t)(n_tri + 3) / 4 * 128 * sizeof(float); }
 
 int sm_count()
 {

@@ -78,10 +78,18 @@ cudaError_t walk_drain(const Args &a, const int *q_in, int round, cudaStream_t s
     const bool nearest = a.opt.order == 1, tree = a.n_tri > 32 * kMaskWords;
     RayState *states = static_cast<RayState *>(a.states);
     LeafJob *leaves = static_cast<LeafJob *>(a.leaves);
-#define DMAP_DRAIN(ST_, TR_, NR_, DP_)                                                                              \
-    wave_walk<ST_, true, TR_, NR_, DP_><<<a.grid, 128, 0, stream>>>(                                     \
-        a.t32, a.t64, a.n_tri, a.assets, a.rays, a.n, a.opt, a.hits, ST_ ? a.stats : nullptr, states, q_in, round, leaves,  \
-        a.counters, a.status, a.rerun)
+    // with its stacks and the entries of more than 164 triangles it passes the
+    // 48 KB that need no opt-in
+    const size_t bytes = entry_bytes(a.n_tri);
+    cudaError_t e = cudaSuccess;
+    auto run = [&](auto *kernel, int64_t *stats) {
+        if (bytes > 20480)
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e == cudaSuccess)
+            kernel<<<a.grid, 128, bytes, stream>>>(a.t32, a.t64, a.n_tri, a.assets, a.rays, a.n, a.opt, a.hits, stats,
+                                                   states, q_in, round, leaves, a.counters, a.status, a.rerun);
+    };
+#define DMAP_DRAIN(ST_, TR_, NR_, DP_) run(wave_walk<ST_, true, TR_, NR_, DP_>, ST_ ? a.stats : nullptr)
 #define DMAP_DRAIN_DEEP(ST_, TR_, NR_)                                                                              \
     (ST_ || a.opt.deep ? DMAP_DRAIN(ST_, TR_, NR_, true) : DMAP_DRAIN(false, TR_, NR_, false))
 #define DMAP_DRAIN_MODE(ST_)                                                                                        \
@@ -94,7 +102,7 @@ cudaError_t walk_drain(const Args &a, const int *q_in, int round, cudaStream_t s
 #undef DMAP_DRAIN_MODE
 #undef DMAP_DRAIN_DEEP
 #undef DMAP_DRAIN
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t filter(const Args &a, int round, cudaStream_t stream)
