@@ -1,11 +1,12 @@
-// Per-triangle setup (one thread per base triangle), in double with the
-// reference's operation order (compiled with -fmad=false):
+// Per-triangle setup (a block per base triangle: one thread but for the height
+// range), in double with the reference's operation order (compiled with
+// -fmad=false):
 //   BaseTriangle general-chart constructor   displaced_surface.cpp:54-91
 //   tangent_frame                             node_bounds.cpp:13-23
 //   UvTriangle                                uv_clip.cpp:10-25
 //   footprint_roots                           descent_sampler.cpp:66-83
 //   DisplacedIntersector roots, tolerance     displaced_intersector.cpp:135-151
-//   triangle_height_range (explicit stack)    node_bounds.cpp:218-249
+//   triangle_height_range (shared stack)      node_bounds.cpp:218-249
 //   triangle_aabb                             node_bounds.cpp:251-269
 // and the FP32 record derived from it, rounded outward where it bounds.
 #include "device_types.cuh"
@@ -138,15 +139,27 @@ __device__ bool init_triangle(TriDev &T, const double *r, bool chart)
     return true;
 }
 
+constexpr int kThreads = 64;
+constexpr int kStack = 1024;
+
+// A cell of the footprint still to visit.
 struct StackCell { int level; int64_t i, j; };
 
-__device__ void setup_one(TriDev &T, const AssetDev &a, unsigned *status)
+struct RangeWalk
+{
+    StackCell cell[kStack];
+    int n, visits;
+    bool capped;
+    double lo[kThreads], hi[kThreads];
+};
+
+// DisplacedIntersector's roots: the block's cells meeting the domain's box, j
+// outer. Returns the footprint's first root in i0, j0.
+__device__ void setup_roots(TriDev &T, const AssetDev &a, int64_t &i0, int64_t &j0)
 {
     int level;
-    int64_t i0, j0;
     footprint_roots(T, a.n_leaf, level, i0, j0);
     T.root_level = level;
-    // DisplacedIntersector roots: the block's cells meeting the domain's box, j outer
     double w = cell_width(a, level);
     int64_t i_lo = (int64_t)floor(T.lo[0] / w), i_hi = (int64_t)ceil(T.hi[0] / w) - 1;
     int64_t j_lo = (int64_t)floor(T.lo[1] / w), j_hi = (int64_t)ceil(T.hi[1] / w) - 1;
@@ -158,38 +171,87 @@ __device__ void setup_one(TriDev &T, const AssetDev &a, unsigned *status)
             ++n;
         }
     T.n_roots = n;
-    // triangle_height_range: depth-first over the footprint, explicit stack
-    double h_min = INFINITY, h_max = -INFINITY;
-    StackCell st[96];
-    int sp = 0;
-    for (int ch = 3; ch >= 0; --ch)
-        st[sp++] = {level, i0 + (ch & 1), j0 + (ch >> 1)};
-    int guard = 0;
-    while (sp > 0) {
-        if (++guard > (1 << 26)) {
-            atomicOr(status, dmapdev::kStatusCapped);
-            break;
-        }
-        StackCell c = st[--sp];
-        double cw = cell_width(a, c.level);
-        v2 cc = {(c.i + 0.5) * cw, (c.j + 0.5) * cw};
-        int ov = classify_square(T, cc, 0.5 * cw);
-        if (ov == OUTSIDE)
-            continue;
-        if (ov == INSIDE || c.level == 0) {
-            double lo, hi;
-            node_hrange(a, c.level, c.i, c.j, lo, hi);
-            h_min = dmin(h_min, lo);
-            h_max = dmax(h_max, hi);
-            continue;
-        }
-        if (sp + 4 > 96) {
-            atomicOr(status, dmapdev::kStatusCapped);
-            break;
-        }
-        for (int ch = 3; ch >= 0; --ch)
-            st[sp++] = {c.level - 1, 2 * c.i + (ch & 1), 2 * c.j + (ch >> 1)};
+}
+
+// triangle_height_range over the footprint: the cells inside the domain, and
+// the leaf cells straddling its edges, fold their height ranges (a minimum
+// and a maximum, so the order of the visits does not matter). The block takes
+// as many cells off the stack at once as it has threads and the stack has
+// room for their children. One thread's depth-first walk visited the cells of
+// a 1024^2 map's diagonal one load after another: the setup of a quad took
+// 3.2 ms, so it takes 0.11.
+__device__ void height_range(RangeWalk &W, const TriDev &T, const AssetDev &a, int64_t i0, int64_t j0, unsigned *status,
+                             double &h_min, double &h_max)
+{
+    const int tid = threadIdx.x;
+    if (tid < 4)
+        W.cell[tid] = {T.root_level, i0 + (tid & 1), j0 + (tid >> 1)};
+    if (tid == 0) {
+        W.n = 4;
+        W.visits = 0;
+        W.capped = false;
     }
+    double lo_all = INFINITY, hi_all = -INFINITY;
+    __syncthreads();
+    for (;;) {
+        const int n = W.n;
+        if (n == 0 || W.capped)
+            break;
+        // all of them but for a reserve, in which one at a time goes depth
+        // first (three cells wait per level, at most 31 levels)
+        int take = (kStack - 128 - n) / 4;
+        take = take < 1 ? 1 : take < kThreads ? take : kThreads;
+        take = take < n ? take : n;
+        StackCell c = {0, 0, 0};
+        if (tid < take)
+            c = W.cell[n - 1 - tid];
+        __syncthreads();
+        if (tid == 0) {
+            W.n = n - take;
+            W.visits += take;
+            if (W.visits > (1 << 26))
+                W.capped = true;
+        }
+        __syncthreads();
+        if (tid < take) {
+            double cw = cell_width(a, c.level);
+            v2 cc = {(c.i + 0.5) * cw, (c.j + 0.5) * cw};
+            int ov = classify_square(T, cc, 0.5 * cw);
+            if (ov != OUTSIDE && (ov == INSIDE || c.level == 0)) {
+                double lo, hi;
+                node_hrange(a, c.level, c.i, c.j, lo, hi);
+                lo_all = dmin(lo_all, lo);
+                hi_all = dmax(hi_all, hi);
+            } else if (ov != OUTSIDE) {
+                if (T.root_level - c.level >= 30) { // a footprint beyond 2^30 cells a side
+                    W.capped = true;
+                } else {
+                    const int at = atomicAdd(&W.n, 4);
+                    for (int ch = 0; ch < 4; ++ch)
+                        W.cell[at + ch] = {c.level - 1, 2 * c.i + (ch & 1), 2 * c.j + (ch >> 1)};
+                }
+            }
+        }
+        __syncthreads();
+    }
+    W.lo[tid] = lo_all;
+    W.hi[tid] = hi_all;
+    __syncthreads();
+    if (tid == 0) {
+        if (W.capped)
+            atomicOr(status, dmapdev::kStatusCapped);
+        for (int k = 1; k < kThreads; ++k) {
+            lo_all = dmin(lo_all, W.lo[k]);
+            hi_all = dmax(hi_all, W.hi[k]);
+        }
+    }
+    h_min = lo_all;
+    h_max = hi_all;
+}
+
+// triangle_aabb from the height range
+__device__ void setup_box(TriDev &T, double h_min, double h_max)
+{
     T.h_min = h_min;
     T.h_max = h_max;
     // triangle_aabb: three parallelograms
@@ -260,29 +322,41 @@ __device__ void derive32(const TriDev &T, const AssetDev &g, TriDev32 &S)
     S.q22 = (float)dot3(Mv, Mv);
 }
 
-__global__ void setup_kernel(const double *__restrict__ tris, int stride, const int *__restrict__ tri_asset,
-                             const AssetDev *__restrict__ assets, int n_tri, TriDev *out, TriDev32 *out32,
-                             unsigned *status)
+__global__ void __launch_bounds__(kThreads)
+    setup_kernel(const double *__restrict__ tris, int stride, const int *__restrict__ tri_asset,
+                 const AssetDev *__restrict__ assets, int n_tri, TriDev *out, TriDev32 *out32, unsigned *status)
 {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n_tri)
-        return;
-    TriDev T;
-    T.asset = tri_asset[k];
-    T.status = 0;
-    T.inst = 0;
-    T.inst_pad = 0;
-    if (!init_triangle(T, tris + stride * (size_t)k, stride == dmapk::kChartRecord)) {
-        T.status = 1;
-        atomicOr(status, dmapdev::kStatusBadInput);
-        out[k] = T;
-        return;
+    __shared__ TriDev T;
+    __shared__ RangeWalk W;
+    __shared__ int64_t s_root[2];
+    __shared__ bool s_ok;
+    const int k = blockIdx.x;
+    if (threadIdx.x == 0) {
+        T.asset = tri_asset[k];
+        T.status = 0;
+        T.inst = 0;
+        T.inst_pad = 0;
+        s_ok = init_triangle(T, tris + stride * (size_t)k, stride == dmapk::kChartRecord);
+        if (s_ok) {
+            setup_roots(T, assets[T.asset], s_root[0], s_root[1]);
+        } else {
+            T.status = 1;
+            atomicOr(status, dmapdev::kStatusBadInput);
+            out[k] = T;
+        }
     }
-    setup_one(T, assets[T.asset], status);
-    out[k] = T;
-    TriDev32 S;
-    derive32(T, assets[T.asset], S);
-    out32[k] = S;
+    __syncthreads();
+    if (!s_ok)
+        return;
+    double h_min, h_max;
+    height_range(W, T, assets[T.asset], s_root[0], s_root[1], status, h_min, h_max);
+    if (threadIdx.x == 0) {
+        setup_box(T, h_min, h_max);
+        out[k] = T;
+        TriDev32 S;
+        derive32(T, assets[T.asset], S);
+        out32[k] = S;
+    }
 }
 
 } // namespace
@@ -293,9 +367,7 @@ cudaError_t launch_setup(const double *tris_dev, int stride, const int *tri_asse
                          const dmapdev::AssetDev *assets_dev, int n_tri, dmapdev::TriDev *out,
                          dmapdev::TriDev32 *out32, unsigned *status, cudaStream_t stream)
 {
-    int threads = 64;
-    int blocks = (n_tri + threads - 1) / threads;
-    setup_kernel<<<blocks, threads, 0, stream>>>(tris_dev, stride, tri_asset_dev, assets_dev, n_tri, out, out32,
+    setup_kernel<<<n_tri, kThreads, 0, stream>>>(tris_dev, stride, tri_asset_dev, assets_dev, n_tri, out, out32,
                                                  status);
     return cudaGetLastError();
 }
