@@ -144,22 +144,29 @@ dmap_status dmap_asset_create(dmap_context *ctx, const void *values_host, dmap_d
         return s;
     };
     cudaError_t e;
+    // FP64 levels: all of them when they are kept, else those the fold
+    // launches read back, from the first tile's top on (1/256 of the cells;
+    // allocating and freeing all of a 1024^2 map's took 0.4 of 2.3 ms)
+    const bool keep64 = (flags & DMAP_ASSET_KEEP_F64) != 0;
+    const int tile = n < 16 ? n : 16;
+    const int64_t first64 = keep64 ? 0 : d.level_off[__builtin_ctz((unsigned)tile)];
     if ((e = cudaMalloc(&a->nodes, (size_t)pitch * nodes * es)) != cudaSuccess ||
-        (e = cudaMalloc((void **)&a->pyr64, (size_t)cells * 64)) != cudaSuccess ||
+        (e = cudaMalloc((void **)&a->pyr64, (size_t)(cells - first64) * 64)) != cudaSuccess ||
         (e = cudaMalloc((void **)&a->pyr32, (size_t)cells * 32)) != cudaSuccess)
         return cleanup(cuda_fail(ctx, e, "dmap_asset_create: cudaMalloc"));
     if ((e = cudaMemcpy2DAsync(a->nodes, (size_t)pitch * es, values_host, (size_t)nodes * es, (size_t)nodes * es,
                                nodes, cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess)
         return cleanup(cuda_fail(ctx, e, "dmap_asset_create: upload"));
     d.nodes = a->nodes;
-    d.pyr64 = a->pyr64;
+    d.pyr64 = keep64 ? a->pyr64 : nullptr;
     d.pyr32 = a->pyr32;
+    double *const levels64 = a->pyr64 - 8 * first64; // indexed by cell from level 0
 
     // TMA descriptor over the node grid: a (T+1) x box_w tile per CTA.
     EncodeTiledFn enc = encode_tiled();
     if (!enc)
         return cleanup(fail(ctx, DMAP_ERR_CUDA, "dmap_asset_create: cuTensorMapEncodeTiled unavailable"));
-    int T = n < 16 ? n : 16;
+    const int T = tile;
     cuuint32_t box_w = (cuuint32_t)(((T + 1) * es + 15) / 16 * 16 / es);
     CUtensorMap tmap;
     cuuint64_t dims[2] = {(cuuint64_t)nodes, (cuuint64_t)nodes};
@@ -183,10 +190,8 @@ dmap_status dmap_asset_create(dmap_context *ctx, const void *values_host, dmap_d
     if (direct && (e = cudaMalloc(&hull, ((size_t)cells + 32768) * 32)) != cudaSuccess)
         return cleanup(cuda_fail(ctx, e, "dmap_asset_create: cudaMalloc"));
     cudaEventRecord(ev[0], ctx->stream);
-    e = direct ? dmapk::launch_pyramid_direct(d, a->pyr64, a->pyr32, hull, ctx->stream,
-                                              (flags & DMAP_ASSET_KEEP_F64) != 0)
-               : dmapk::launch_pyramid(&tmap, d, T, a->pyr64, a->pyr32, ctx->status_dev, ctx->stream,
-                                       (flags & DMAP_ASSET_KEEP_F64) != 0);
+    e = direct ? dmapk::launch_pyramid_direct(d, levels64, a->pyr32, hull, ctx->stream, keep64)
+               : dmapk::launch_pyramid(&tmap, d, T, levels64, a->pyr32, ctx->status_dev, ctx->stream, keep64);
     cudaEventRecord(ev[1], ctx->stream);
     if (e != cudaSuccess) {
         cudaEventDestroy(ev[0]);
@@ -215,10 +220,9 @@ dmap_status dmap_asset_create(dmap_context *ctx, const void *values_host, dmap_d
     cudaFree(hull);
     if (s != DMAP_OK)
         return cleanup(s);
-    if (!(flags & DMAP_ASSET_KEEP_F64)) {
+    if (!keep64) {
         cudaFree(a->pyr64);
         a->pyr64 = nullptr;
-        d.pyr64 = nullptr;
     }
     a->bytes = (size_t)pitch * nodes * es + (size_t)cells * 32 + (a->pyr64 ? (size_t)cells * 64 : 0);
     *out = a;
