@@ -14,23 +14,26 @@ namespace d32
 // leave as the entry / exit bounds: t0 is a lower bound of the exact entry
 // of any box inside this one, t1 an upper bound of its exit. False when an
 // axis the ray does not move along misses the box.
+__device__ __forceinline__ bool box_slab(float box_lo, float box_hi, float o, float d, float inv, float &t0, float &t1)
+{
+    float bmag = fmaxf(fabsf(box_lo), fabsf(box_hi));
+    float pad = ru_mul(2.0f * G, ru_add(ru_fma(2.0f, fabsf(o), bmag), 1.0f));
+    float lo = __fsub_rd(box_lo, pad), hi = __fadd_ru(box_hi, pad);
+    if (d == 0.0f)
+        return !(o < lo || o > hi);
+    float ta = (lo - o) * inv, tb = (hi - o) * inv;
+    t0 = fmaxf(t0, fminf(ta, tb));
+    t1 = fminf(t1, fmaxf(ta, tb));
+    return true;
+}
+
 __device__ __forceinline__ bool box_slabs(const float *box_lo, const float *box_hi, const float *of, const float *df,
                                           const float *invf, float &t0, float &t1)
 {
     bool ok = true;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        float bmag = fmaxf(fabsf(box_lo[a]), fabsf(box_hi[a]));
-        float pad = ru_mul(2.0f * G, ru_add(ru_fma(2.0f, fabsf(of[a]), bmag), 1.0f));
-        float lo = __fsub_rd(box_lo[a], pad), hi = __fadd_ru(box_hi[a], pad);
-        if (df[a] != 0.0f) {
-            float ta = (lo - of[a]) * invf[a], tb = (hi - of[a]) * invf[a];
-            t0 = fmaxf(t0, fminf(ta, tb));
-            t1 = fminf(t1, fmaxf(ta, tb));
-        } else if (of[a] < lo || of[a] > hi) {
-            ok = false;
-        }
-    }
+    for (int a = 0; a < 3; ++a)
+        ok = box_slab(box_lo[a], box_hi[a], of[a], df[a], invf[a], t0, t1) && ok;
     return ok;
 }
 

@@ -575,14 +575,11 @@ struct Span
 __device__ __noinline__ Span box_span(const float *box, int stride, const RaySlot &S, float t0, float t1,
                                       float wide = 1.0f, float t_lo = 0.0f)
 {
-    float lo[3], hi[3];
+    Span r = {t0, t1, true};
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        lo[c] = box[c * stride];
-        hi[c] = box[(3 + c) * stride];
-    }
-    Span r = {t0, t1, false};
-    r.ok = box_slabs(lo, hi, S.of, S.df, S.invf, r.t0, r.t1) && !misses(r.t0, r.t1, wide, t_lo);
+    for (int c = 0; c < 3; ++c)
+        r.ok = box_slab(box[c * stride], box[(3 + c) * stride], S.of[c], S.df[c], S.invf[c], r.t0, r.t1) && r.ok;
+    r.ok = r.ok && !misses(r.t0, r.t1, wide, t_lo);
     return r;
 }
 
@@ -697,6 +694,9 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
     // the rays in work and those the warp has fetched ahead
     constexpr int kRaySlots = 16, kRayBatch = 8; // per warp: eight in work, eight ahead
     __shared__ RaySlot s_ray[4][kRaySlots];
+    // the quads' rays in their triangles' frames: per axis origin, direction,
+    // its reciprocal, widening (Ray32)
+    __shared__ float4 s_frame[32][3];
     // the last walk: the leaf search's stacks, per quad
     __shared__ double s_stack[INLINE_LEAF ? 32 : 1][INLINE_LEAF ? lq::kStack * sizeof(lq::P64::Ent) / 8 : 1];
     // items of this round: every ray in round 0, else the resume queue
@@ -733,7 +733,7 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
     d32::NearBuf nbuf;
     nbuf.n = -1;
     nbuf.pos = 0;
-    Ray32 r;
+    float4 *const frame = s_frame[threadIdx.x >> 2];
     const float *pyr = nullptr;
     Cell32 cur = {0, 0, 0};
     CellBits<DEEP> todo = {0ull, 0ull}, dom = {0ull, 0ull}; // cells that passed; cells in the domain, not yet gone past
@@ -796,15 +796,15 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
     // the ray transform into triangle T's tangent frame, a row per lane
     auto enter_frame = [&](const TriDev32 &T, const double *o, const double *d, float t_far) {
         const unsigned quad = 0xfu << lead;
-        float ro, rd, e;
-        tangent_row(T, sub < 3 ? sub : 0, o, d, t_far, ro, rd, e);
-        const float inv = rd != 0.0f ? __frcp_rn(rd) : 0.0f;
-        r.ox = __shfl_sync(quad, ro, lead), r.oy = __shfl_sync(quad, ro, lead + 1), r.oz = __shfl_sync(quad, ro, lead + 2);
-        r.dx = __shfl_sync(quad, rd, lead), r.dy = __shfl_sync(quad, rd, lead + 1), r.dz = __shfl_sync(quad, rd, lead + 2);
-        r.ix = __shfl_sync(quad, inv, lead), r.iy = __shfl_sync(quad, inv, lead + 1), r.iz = __shfl_sync(quad, inv, lead + 2);
-        r.ex = __shfl_sync(quad, e, lead), r.ey = __shfl_sync(quad, e, lead + 1), r.ez = __shfl_sync(quad, e, lead + 2);
-        si = r.dx < 0.0f;
-        sj = r.dy < 0.0f;
+        if (sub < 3) {
+            float4 f;
+            tangent_row(T, sub, o, d, t_far, f.x, f.y, f.w);
+            f.z = f.y != 0.0f ? __frcp_rn(f.y) : 0.0f;
+            frame[sub] = f;
+        }
+        __syncwarp(quad);
+        si = frame[0].y < 0.0f;
+        sj = frame[1].y < 0.0f;
         pyr = T.pyr32;
     };
 
@@ -1275,6 +1275,8 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
             const int cj = roots ? T.roots_j[sub] : 2 * pj + ((sub & 1) ^ sj);
             const float w = pow2f(tl - W.log2n);
             in = square_meets_domain(W, ((float)ci + 0.5f) * w, ((float)cj + 0.5f) * w, 0.5f * w);
+            const float4 fx = frame[0], fy = frame[1], fz = frame[2];
+            const Ray32 r = {fx.x, fy.x, fz.x, fx.y, fy.y, fz.y, fx.z, fy.z, fz.z, fx.w, fy.w, fz.w};
             if (in)
                 pass = node_test32(W, pyr, r, tl, ci, cj, tmin_f, tmax_f, opt.bound, opt.slab_max_level);
         }
