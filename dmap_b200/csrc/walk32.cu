@@ -21,10 +21,18 @@ cudaError_t walk_round(const Args &a, const int *q_in, int round, cudaStream_t s
     const bool nearest = a.opt.order == 1, tree = a.n_tri > 32 * kMaskWords;
     RayState *states = static_cast<RayState *>(a.states);
     LeafJob *leaves = static_cast<LeafJob *>(a.leaves);
-#define DMAP_ROUND(ST_, TR_, NR_, DP_)                                                                              \
-    wave_walk<ST_, false, TR_, NR_, DP_><<<a.grid, 128, entry_bytes(a.n_tri), stream>>>(                                     \
-        a.t32, a.t64, a.n_tri, a.assets, a.rays, a.n, a.opt, a.hits, ST_ ? a.stats : nullptr, states, q_in, round, leaves,  \
-        a.counters, a.status, a.rerun)
+    // the entries of more than 252 triangles pass the 48 KB of shared memory
+    // that need no opt-in
+    const size_t bytes = entry_bytes(a.n_tri);
+    cudaError_t e = cudaSuccess;
+    auto run = [&](auto *kernel, int64_t *stats) {
+        if (bytes > 32256)
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e == cudaSuccess)
+            kernel<<<a.grid, 128, bytes, stream>>>(a.t32, a.t64, a.n_tri, a.assets, a.rays, a.n, a.opt, a.hits, stats,
+                                                   states, q_in, round, leaves, a.counters, a.status, a.rerun);
+    };
+#define DMAP_ROUND(ST_, TR_, NR_, DP_) run(wave_walk<ST_, false, TR_, NR_, DP_>, ST_ ? a.stats : nullptr)
 #define DMAP_ROUND_DEEP(ST_, TR_, NR_)                                                                              \
     (ST_ || a.opt.deep ? DMAP_ROUND(ST_, TR_, NR_, true) : DMAP_ROUND(false, TR_, NR_, false))
 #define DMAP_ROUND_MODE(ST_)                                                                                        \
@@ -37,7 +45,7 @@ cudaError_t walk_round(const Args &a, const int *q_in, int round, cudaStream_t s
 #undef DMAP_ROUND_MODE
 #undef DMAP_ROUND_DEEP
 #undef DMAP_ROUND
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 // One query: the simple schedule's single launch, or the wavefront's rounds
