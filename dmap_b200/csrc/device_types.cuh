@@ -57,9 +57,8 @@ struct TriDev
 };
 
 // The FP32 record: what the walk reads, plus the FP64 frame origin and
-// matrix for the per-ray transform. The node test and the domain test read
-// the first 128 bytes (one cache line) as eight 16-byte loads
-// (f32_node.cuh:load_walk).
+// matrix for the per-ray transform. The node test and the walk's domain test
+// read nine 16-byte words of it (f32_node.cuh:load_walk).
 struct alignas(128) TriDev32
 {
     // The interpolated normal in tangent space, A N(s,t) = a0 + s au + t av,
@@ -70,9 +69,17 @@ struct alignas(128) TriDev32
     float qc, q1, q2, q11, q12, q22;
     float lo[2], hi[2];    // texture-space box of the domain, outward
     float un[3][2], ud[3]; // domain edges (exact for dyadic texture coordinates)
-    int log2n;             // the asset's pyramid: 2^log2n leaf cells per side
+    float pad0;
+    // Bounds over the whole domain of what the node test rounds, so that it
+    // adds constants (X, Y: the largest |s|, |t| of the domain's box, G = 2^-20):
+    float nerr[3]; // G (|a0| + X |au| + Y |av|) per axis
+    float qerr;    // 2 G of the same sum of |N|^2's terms
+    float udm[3];  // ud less the domain test's rounding over the footprint's cells
+    int log2n;     // the asset's pyramid: 2^log2n leaf cells per side
+    float perr[3]; // 2 G (X, Y, 0): the base point's roundings
+    float pad1;
     const float *pyr32;
-    int root_level, n_roots, asset, pad;
+    int root_level, n_roots, asset, pad2;
     int roots_i[4], roots_j[4];
     double A[3][3];        // to_tangent in double for the ray transform
     double q0[3];

@@ -62,21 +62,22 @@ __device__ __forceinline__ Node32 fetch_node(const float *pyr32, int L, int leve
     return n;
 }
 
-// The first 128 bytes of a triangle's FP32 record, loaded as eight 16-byte
-// words: what the node test and the domain test read.
+// What the node test and the walk's domain test read of a triangle's FP32
+// record, loaded as nine 16-byte words.
 struct Walk32
 {
     float4 n[3]; // per axis: a0, au, av, rowsum
     float qc, q1, q2, q11, q12, q22;
     float lox, loy, hix, hiy;
-    float ux[3], uy[3], ud[3];
+    float ux[3], uy[3], udm[3];
+    float nerr[3], qerr;
     int log2n;
 };
 
 __device__ __forceinline__ Walk32 load_walk(const TriDev32 &T)
 {
     const float4 *p = reinterpret_cast<const float4 *>(&T);
-    const float4 a = __ldg(p + 3), b = __ldg(p + 4), c = __ldg(p + 5), d = __ldg(p + 6), e = __ldg(p + 7);
+    const float4 a = __ldg(p + 3), b = __ldg(p + 4), c = __ldg(p + 5), d = __ldg(p + 6), f = __ldg(p + 8), g = __ldg(p + 9);
     Walk32 w;
     w.n[0] = __ldg(p);
     w.n[1] = __ldg(p + 1);
@@ -85,8 +86,9 @@ __device__ __forceinline__ Walk32 load_walk(const TriDev32 &T)
     w.q12 = b.x, w.q22 = b.y;
     w.lox = b.z, w.loy = b.w, w.hix = c.x, w.hiy = c.y;
     w.ux[0] = c.z, w.uy[0] = c.w, w.ux[1] = d.x, w.uy[1] = d.y, w.ux[2] = d.z, w.uy[2] = d.w;
-    w.ud[0] = e.x, w.ud[1] = e.y, w.ud[2] = e.z;
-    w.log2n = __float_as_int(e.w);
+    w.nerr[0] = f.x, w.nerr[1] = f.y, w.nerr[2] = f.z, w.qerr = f.w;
+    w.udm[0] = g.x, w.udm[1] = g.y, w.udm[2] = g.z;
+    w.log2n = __float_as_int(g.w);
     return w;
 }
 
@@ -121,16 +123,29 @@ __device__ __forceinline__ void cell_next(Cell32 &c, int si, int sj, int root_le
 }
 
 // classify_square (uv_clip.cpp:27-44) reporting Outside only when the
-// separation exceeds the rounding of the test.
-__device__ __forceinline__ bool square_meets_domain(const Walk32 &T, float cx, float cy, float s)
+// separation exceeds the rounding of the test: of a footprint's cell, with
+// the bound of that rounding in udm, ...
+__device__ __forceinline__ bool cell_meets_domain(const Walk32 &T, float cx, float cy, float s)
 {
     if (cx + s <= T.lox || cx - s >= T.hix || cy + s <= T.loy || cy - s >= T.hiy)
         return false;
+    bool out = false;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        out = out || __fmaf_rn(fabsf(T.ux[k]) + fabsf(T.uy[k]), s, __fmaf_rn(T.uy[k], cy, T.ux[k] * cx)) <= T.udm[k];
+    return !out;
+}
+
+// ... and of a leaf's sub-square, with the bound taken where it is.
+__device__ __forceinline__ bool square_meets_domain(const TriDev32 &T, float cx, float cy, float s)
+{
+    if (cx + s <= T.lo[0] || cx - s >= T.hi[0] || cy + s <= T.lo[1] || cy - s >= T.hi[1])
+        return false;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        float proj = __fmaf_rn(T.uy[k], cy, T.ux[k] * cx);
-        float ext = (fabsf(T.ux[k]) + fabsf(T.uy[k])) * s;
-        float slack = G * (fabsf(T.ux[k] * cx) + fabsf(T.uy[k] * cy) + fabsf(T.ud[k]) + ext);
+        float proj = __fmaf_rn(T.un[k][1], cy, T.un[k][0] * cx);
+        float ext = (fabsf(T.un[k][0]) + fabsf(T.un[k][1])) * s;
+        float slack = G * (fabsf(T.un[k][0] * cx) + fabsf(T.un[k][1] * cy) + fabsf(T.ud[k]) + ext);
         if (proj + ext + slack <= T.ud[k])
             return false;
     }
@@ -168,22 +183,20 @@ __device__ __forceinline__ void clip_axis(float o, float d, float inv, float lo,
 
 // The range of 1/|N| over the rectangle [cx +- hx] x [cy +- hy], with
 // |N(s,t)|^2 = qc + 2 s q1 + 2 t q2 + s^2 q11 + 2 s t q12 + t^2 q22, as
-// midpoint rm and radius rr; false when |N| may vanish there.
+// midpoint rm and radius rr; false when |N| may vanish there. The roundings
+// of the centre value and of the spread are at most some ten units in the
+// last place of the sum of the terms' magnitudes, whose bound over the domain
+// gives qerr.
 __device__ __forceinline__ bool inv_norm_range(const Walk32 &T, float cx, float cy, float hx, float hy, float &rm,
                                                float &rr)
 {
-    float gs = 2.0f * hx * __fmaf_rn(cy, T.q12, __fmaf_rn(cx, T.q11, T.q1));
-    float gt = 2.0f * hy * __fmaf_rn(cy, T.q22, __fmaf_rn(cx, T.q12, T.q2));
-    float sx = cx * cx, sy = cy * cy, sxy = cx * cy;
-    float qv = __fmaf_rn(2.0f * cy, T.q2, __fmaf_rn(2.0f * cx, T.q1, T.qc));
-    qv = __fmaf_rn(sy, T.q22, __fmaf_rn(2.0f * sxy, T.q12, __fmaf_rn(sx, T.q11, qv)));
-    float mag = ru_add(ru_add(fabsf(T.qc), ru_mul(2.0f, ru_add(fabsf(cx * T.q1), fabsf(cy * T.q2)))),
-                       ru_add(ru_add(sx * fabsf(T.q11), sy * fabsf(T.q22)), 2.0f * fabsf(sxy * T.q12)));
-    float quad = ru_add(ru_mul(hx * hx, fabsf(T.q11)), ru_mul(hy * hy, fabsf(T.q22)));
-    float spread = ru_add(ru_add(fabsf(gs), fabsf(gt)), ru_mul(2.0f, ru_mul(ru_mul(hx, hy), fabsf(T.q12))));
-    float err = ru_mul(G, ru_add(ru_add(mag, spread), quad));
-    float q_lo = __fsub_rd(__fsub_rd(qv, spread), err);
-    float q_hi = ru_add(ru_add(ru_add(qv, spread), err), quad);
+    const float gs = __fmaf_rn(cy, T.q12, __fmaf_rn(cx, T.q11, T.q1));
+    const float gt = __fmaf_rn(cy, T.q22, __fmaf_rn(cx, T.q12, T.q2));
+    const float qv = __fmaf_rn(cy, T.q2 + gt, __fmaf_rn(cx, T.q1 + gs, T.qc));
+    const float hx2 = hx + hx, hy2 = hy + hy;
+    const float quad = ru_fma(hx * hx, fabsf(T.q11), ru_mul(hy * hy, fabsf(T.q22)));
+    const float spread = ru_add(ru_fma(hx2, ru_fma(hy, fabsf(T.q12), fabsf(gs)), ru_mul(hy2, fabsf(gt))), T.qerr);
+    const float q_lo = __fsub_rd(qv, spread), q_hi = ru_add(ru_add(qv, spread), quad);
     if (!(q_lo > 0.0f) || !(q_hi < INFINITY))
         return false;
     const float up = 1.0f + 9.5367431640625e-07f, dn = 1.0f - 9.5367431640625e-07f;
@@ -195,42 +208,33 @@ __device__ __forceinline__ bool inv_norm_range(const Walk32 &T, float cx, float 
 
 // One component of the tangent normal's enclosure m_k = (A N)_k / |N|: the
 // affine form of (A N)_k = a0 + s au + t av over the rectangle (its
-// coefficients rounded from double, their rounding in k0) times the interval
-// rm +- rr. Then the box coordinate p_k + h m_k with h = mid +- hh and the
-// base point's form (pc, pa, pb), hulled outward and widened by the ray's E.
-__device__ __forceinline__ void box_axis(float a0, float au, float av, float cx, float cy, float hx, float hy,
-                                         bool ok, float rm, float rr, float rowsum, float mid, float hh, float pc,
-                                         float pa, float pb, float E, float &lo, float &hi, float &m_lo, float &m_hi)
+// coefficients rounded from double, their rounding and the evaluation's in
+// nerr) times the interval rm +- rr. Then the box coordinate p_k + h m_k with
+// h = mid +- hh and the base point's form (pc, pa, pb), hulled outward and
+// widened by E: the ray's own rounding and the base point's (perr).
+// With s1 = |nc| + |na| + |nb|: m = c + a eu + b ev + rho, |rho| <= k =
+// rr (s1 + nerr) + rm (G s1 + nerr), |c| + |a| + |b| + k <= V = rm' s1 + k,
+// rm' = rm (1 + G); h m + p has the remainder |mid| (k + G V) + hh V.
+__device__ __forceinline__ void box_axis(const float4 &n, float nerr, float cx, float cy, float hx, float hy, bool ok,
+                                         float rm, float rmu, float rr, float mid, float hh, float pc, float pa,
+                                         float pb, float E, float &lo, float &hi, float &mc, float &mh)
 {
-    float c, a, b, k;
-    if (ok) {
-        float tu = cx * au, tv = cy * av;
-        float nc = __fmaf_rn(cy, av, __fmaf_rn(cx, au, a0));
-        float na = hx * au, nb = hy * av;
-        float k0 = ru_mul(G, ru_add(mag3(a0, tu, tv), ru_add(fabsf(na), fabsf(nb))));
-        c = rm * nc;
-        a = rm * na;
-        b = rm * nb;
-        k = ru_fma(G, mag3(c, a, b), ru_fma(rr, ru_add(mag3(nc, na, nb), k0), ru_mul(rm, k0)));
-    } else {
-        // |N| can vanish over the rectangle: a unit normal maps into |m_k| <= sum_j |A_kj|
-        c = a = b = 0.0f;
-        k = rowsum;
-    }
-    float half = ru_add(ru_add(fabsf(a), fabsf(b)), k);
-    m_lo = __fsub_rd(c, half);
-    m_hi = __fadd_ru(c, half);
-    // h m (affine_form.cpp:35-47 with h = mid +- hh), then + p
-    float sc = mid * c, sa = mid * a, sb = mid * b;
-    float sk = ru_fma(G, mag3(sc, sa, sb), ru_fma(hh, ru_add(mag3(c, a, b), k), ru_mul(fabsf(mid), k)));
-    float tc = sc + pc, ta = sa + pa, tb = sb + pb;
-    sk = ru_fma(G, mag3(tc, ta, tb), sk);
-    float e = ru_add(ru_add(ru_add(fabsf(ta), fabsf(tb)), sk), E);
-    lo = __fsub_rd(tc, e);
-    hi = __fadd_ru(tc, e);
-    float gw = ru_mul(G, fmaxf(fabsf(lo), fabsf(hi))); // the clip's own rounding
-    lo = __fsub_rd(lo, gw);
-    hi = __fadd_ru(hi, gw);
+    const float nc = __fmaf_rn(cy, n.z, __fmaf_rn(cx, n.y, n.x));
+    const float na = hx * n.y, nb = hy * n.z;
+    const float s1 = ru_add(ru_add(fabsf(na), fabsf(nb)), fabsf(nc));
+    const float c = rm * nc, a = rm * na, b = rm * nb;
+    float k = ru_fma(rr, ru_add(s1, nerr), ru_mul(rm, ru_fma(G, s1, nerr)));
+    // |N| can vanish over the rectangle (rm = rr = 0): a unit normal maps into |m_k| <= sum_j |A_kj|
+    k = ok ? k : n.w;
+    const float V = ru_fma(rmu, s1, k);
+    mc = c;
+    mh = ru_add(ru_add(fabsf(a), fabsf(b)), k);
+    const float tc = __fmaf_rn(mid, c, pc), ta = __fmaf_rn(mid, a, pa), tb = __fmaf_rn(mid, b, pb);
+    const float sk = ru_fma(hh, V, ru_fma(fabsf(mid), ru_fma(G, V, k), E));
+    const float e = ru_add(ru_add(fabsf(ta), fabsf(tb)), sk);
+    const float w = ru_fma(G, ru_add(fabsf(tc), e), e); // and the clip's own rounding
+    lo = __fsub_rd(tc, w);
+    hi = __fadd_ru(tc, w);
 }
 
 // a / b as a product with the hardware's reciprocal (rcp.approx: within 1
@@ -255,7 +259,11 @@ __device__ __forceinline__ float quot_dn(float a, float b)
 }
 
 // The node test of one cell (node_bounds.cpp:83-211): the box, and at levels
-// <= slab_max_level the slab, both enclosing their double counterparts.
+// <= slab_max_level the slab, both enclosing their double counterparts. Its
+// roundings are bounded by constants of the triangle where a bound over the
+// domain is as good as one at the cell (a box coordinate took 52 operations
+// with every magnitude summed, 33 so: walk rounds of 2.80M rays on 96 x
+// 2048^2 maps 14.6 -> 13.6 ms).
 __device__ __forceinline__ bool node_test32(const Walk32 &T, const float *pyr32, const Ray32 &r, int level, int i,
                                             int j, float t_min, float t_max, int bound, int slab_max_level)
 {
@@ -269,15 +277,13 @@ __device__ __forceinline__ bool node_test32(const Walk32 &T, const float *pyr32,
     float hy = fmaxf(fmaxf(__fsub_ru(rhy, cy), __fsub_ru(cy, rly)), 0.0f);
     float rm = 0.0f, rr = 0.0f;
     bool ok = inv_norm_range(T, cx, cy, hx, hy, rm, rr);
+    const float rmu = ru_mul(rm, 1.0f + G);
     float mid = 0.5f * (n.mn + n.mx);
     float hh = fmaxf(__fsub_ru(n.mx, mid), __fsub_ru(mid, n.mn));
-    float lx, hx_, ly, hy_, lz, hz, mxl, mxh, myl, myh, mzl, mzh;
-    box_axis(T.n[0].x, T.n[0].y, T.n[0].z, cx, cy, hx, hy, ok, rm, rr, T.n[0].w, mid, hh, cx, hx, 0.0f, r.ex, lx,
-             hx_, mxl, mxh);
-    box_axis(T.n[1].x, T.n[1].y, T.n[1].z, cx, cy, hx, hy, ok, rm, rr, T.n[1].w, mid, hh, cy, 0.0f, hy, r.ey, ly,
-             hy_, myl, myh);
-    box_axis(T.n[2].x, T.n[2].y, T.n[2].z, cx, cy, hx, hy, ok, rm, rr, T.n[2].w, mid, hh, 0.0f, 0.0f, 0.0f, r.ez,
-             lz, hz, mzl, mzh);
+    float lx, hx_, ly, hy_, lz, hz, mxc, mxh, myc, myh, mzc, mzh;
+    box_axis(T.n[0], T.nerr[0], cx, cy, hx, hy, ok, rm, rmu, rr, mid, hh, cx, hx, 0.0f, r.ex, lx, hx_, mxc, mxh);
+    box_axis(T.n[1], T.nerr[1], cx, cy, hx, hy, ok, rm, rmu, rr, mid, hh, cy, 0.0f, hy, r.ey, ly, hy_, myc, myh);
+    box_axis(T.n[2], T.nerr[2], cx, cy, hx, hy, ok, rm, rmu, rr, mid, hh, 0.0f, 0.0f, 0.0f, r.ez, lz, hz, mzc, mzh);
     bool read_slab = level <= slab_max_level;
     float b0 = t_min, b1 = t_max;
     if (bound != 1 || !read_slab) {
@@ -297,7 +303,8 @@ __device__ __forceinline__ bool node_test32(const Walk32 &T, const float *pyr32,
     clip_axis(r.oy, r.dy, r.iy, ly, hy_, c0, c1, okc);
     if (!okc || c0 > c1 + tol32(fmaxf(fabsf(c0), fabsf(c1))))
         return false;
-    Iv mx = {mxl, mxh}, my = {myl, myh}, mz = {mzl, mzh};
+    Iv mx = {__fsub_rd(mxc, mxh), __fadd_ru(mxc, mxh)}, my = {__fsub_rd(myc, myh), __fadd_ru(myc, myh)},
+       mz = {__fsub_rd(mzc, mzh), __fadd_ru(mzc, mzh)};
     Iv A = iv_add(iv_add(Iv{1.0f, 1.0f}, iv_scale(n.gu, mx)), iv_scale(n.gv, my));
     Iv B = iv_scale(-n.gu, mz), C = iv_scale(-n.gv, mz);
     float p1lo = rd_mul(n.gu, u0), p1hi = ru_mul(n.gu, u0), p2lo = rd_mul(n.gv, v0), p2hi = ru_mul(n.gv, v0);

@@ -153,7 +153,7 @@ __device__ inline bool sub_square_bound32(const TriDev32 &T32, const Leaf32 &L, 
 {
     using namespace d32;
     float wf = (float)L.w;
-    if (!square_meets_domain(load_walk(T32), (float)L.lo_s + wf * a, (float)L.lo_t + wf * b, wf * rho))
+    if (!square_meets_domain(T32, (float)L.lo_s + wf * a, (float)L.lo_t + wf * b, wf * rho))
         return false;
     const float al = 2.0f * a - 1.0f, be = 2.0f * b - 1.0f, r = 2.0f * rho;
     // the height's deviation from h_mid over the sub-square

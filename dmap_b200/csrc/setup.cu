@@ -301,7 +301,8 @@ __device__ void derive32(const TriDev &T, const AssetDev &g, TriDev32 &S)
     S.root_level = T.root_level;
     S.n_roots = T.n_roots;
     S.asset = T.asset;
-    S.pad = 0;
+    S.pad0 = S.pad1 = 0.0f;
+    S.pad2 = 0;
     for (int k = 0; k < 4; ++k) {
         S.roots_i[k] = T.roots_i[k];
         S.roots_j[k] = T.roots_j[k];
@@ -320,6 +321,25 @@ __device__ void derive32(const TriDev &T, const AssetDev &g, TriDev32 &S)
     S.q11 = (float)dot3(Mu, Mu);
     S.q12 = (float)dot3(Mu, Mv);
     S.q22 = (float)dot3(Mv, Mv);
+    // the node test's rounding bounds over the domain (f32_node.cuh), each
+    // rounded up
+    const double G = 9.5367431640625e-07;
+    const double X = fmax(fabs((double)S.lo[0]), fabs((double)S.hi[0])) * (1.0 + G);
+    const double Y = fmax(fabs((double)S.lo[1]), fabs((double)S.hi[1])) * (1.0 + G);
+    for (int a = 0; a < 3; ++a)
+        S.nerr[a] = fup(G * (fabs(comp(a0, a)) + (X * fabs(comp(au, a)) + Y * fabs(comp(av, a)))) * (1.0 + G));
+    const double q = fabs(dot3(m0, m0)) + 2.0 * (X * fabs(dot3(m0, Mu)) + Y * fabs(dot3(m0, Mv))) +
+                     (X * X * dot3(Mu, Mu) + Y * Y * dot3(Mv, Mv)) + 2.0 * X * Y * fabs(dot3(Mu, Mv));
+    S.qerr = fup(2.0 * G * q * (1.0 + G));
+    S.perr[0] = fup(2.0 * G * X);
+    S.perr[1] = fup(2.0 * G * Y);
+    S.perr[2] = 0.0f;
+    // a footprint's cell reaches at most two root widths past the domain
+    const double w = cell_width(g, T.root_level);
+    for (int k = 0; k < 3; ++k) {
+        const double ux = fabs(T.un[k][0]), uy = fabs(T.un[k][1]);
+        S.udm[k] = fdown(T.ud[k] - G * (ux * (X + 3.0 * w) + uy * (Y + 3.0 * w) + fabs(T.ud[k])));
+    }
 }
 
 __global__ void __launch_bounds__(kThreads)

@@ -97,7 +97,7 @@ __device__ __forceinline__ void tangent_row(const TriDev32 &T, int a, const doub
     const float um = fmaxf(fmaxf(fabsf((float)u0), fabsf((float)u1)), fabsf((float)u2));
     const float dm = fmaxf(fmaxf(fabsf((float)d0), fabsf((float)d1)), fabsf((float)d2));
     const float sum = ru_mul(__double2float_ru(fabs(A0) + fabs(A1) + fabs(A2)), ru_fma(t_far, dm, um));
-    e = ru_fma(0x1p-22f, ru_fma(t_far, fabsf(rd), fabsf(ro)), ru_mul(0x1.1p-40f, sum));
+    e = ru_add(ru_fma(0x1p-22f, ru_fma(t_far, fabsf(rd), fabsf(ro)), ru_mul(0x1.1p-40f, sum)), T.perr[a]);
 }
 
 __device__ __forceinline__ void tangent_ray(const TriDev32 &T, const double *o, const double *d, float t_far,
@@ -185,7 +185,7 @@ __device__ bool triangle_walk32(const TriDev32 &T, const TriDev &T64, const Asse
                 break;
             }
             float w = pow2f(cur.level - W.log2n);
-            if (!square_meets_domain(W, ((float)cur.i + 0.5f) * w, ((float)cur.j + 0.5f) * w, 0.5f * w)) {
+            if (!cell_meets_domain(W, ((float)cur.i + 0.5f) * w, ((float)cur.j + 0.5f) * w, 0.5f * w)) {
                 cell_next(cur, si, sj, T.root_level);
                 continue;
             }
@@ -1274,7 +1274,7 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
             const int ci = roots ? T.roots_i[sub] : 2 * pi + ((sub >> 1) ^ si);
             const int cj = roots ? T.roots_j[sub] : 2 * pj + ((sub & 1) ^ sj);
             const float w = pow2f(tl - W.log2n);
-            in = square_meets_domain(W, ((float)ci + 0.5f) * w, ((float)cj + 0.5f) * w, 0.5f * w);
+            in = cell_meets_domain(W, ((float)ci + 0.5f) * w, ((float)cj + 0.5f) * w, 0.5f * w);
             const float4 fx = frame[0], fy = frame[1], fz = frame[2];
             const Ray32 r = {fx.x, fy.x, fz.x, fx.y, fy.y, fz.y, fx.z, fy.z, fz.z, fx.w, fy.w, fz.w};
             if (in)
