@@ -1306,8 +1306,8 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
 // cells left goes back to the resume queue.
 //
 // The leaf setups (some 800 double operations each) are made by the warp for
-// eight jobs at a time, a lane per cell, ahead of the quads that take them:
-// shared memory holds the setups of the cells in work and of those made
+// up to sixteen jobs at a time, a lane per cell, ahead of the quads that take
+// them: shared memory holds the setups of the cells in work and of those made
 // ready, up to 32 a warp, and the search reads them there (in registers they
 // spilled). Newton runs wait until DMAP_NEWTON_QUADS of a warp's quads have
 // some, and the hit records of the roots found (some 200 double operations
@@ -1315,10 +1315,11 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
 // making its own setups and records as they came, with one or two of the
 // warp's lanes in it, spent most of the kernel there. Leaf rounds of 2.80M
 // rays on the sphere of 96 x 2048^2 maps: a lane per job 9.1 ms, quads 19.7,
-// with batched setups 15.1, batched Newton runs and records 10.0, setups in
-// shared memory 8.1; of 20,011 rays on 512^2 maps 0.72 -> 0.27 ms. The kernel
-// issues in 22% of its cycles at 3 warps per scheduler, half of its stalls
-// instruction fetch.
+// with setups of eight jobs at a time 15.1, batched Newton runs and records
+// 10.0, setups in shared memory 8.1, less code around the ray's load 7.0,
+// setups of sixteen jobs and 32 records at a time 5.8; of 20,011 rays on
+// 512^2 maps 0.72 -> 0.27 ms. The kernel issues in a quarter of its cycles at
+// 3 warps per scheduler; instruction fetch and loads hold it up about alike.
 // Resident CTAs per SM the leaf kernels are compiled for: 6 for the FP32 leaf
 // (168 registers; 5, 7 and 8 are 1-12% slower), 4 for the FP64 leaf.
 #ifndef DMAP_LEAF32_MIN_BLOCKS
@@ -1327,9 +1328,10 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
 #ifndef DMAP_LEAF_MIN_BLOCKS
 #define DMAP_LEAF_MIN_BLOCKS 4
 #endif
-// Quads of a warp with Newton runs waiting before the warp makes them.
+// Quads of a warp with Newton runs waiting before the warp makes them (1M
+// shadow rays, leaf rounds at 4 / 5 / 6 / 7: 4.05 / 3.96 / 3.89 / 3.90 ms).
 #ifndef DMAP_NEWTON_QUADS
-#define DMAP_NEWTON_QUADS 4
+#define DMAP_NEWTON_QUADS 6
 #endif
 constexpr int kLeafThreads = 64;
 constexpr int kLeafBlocks = DMAP_LEAF32_MIN_BLOCKS;
@@ -1346,9 +1348,10 @@ __global__ void __launch_bounds__(kLeafThreads,
     typedef typename P::Ent Ent;
     typedef typename P::Bound Bound;
     enum : int { NEED = 0, SEARCH = 1, NEWTON = 2, DONE = 3 };
-    constexpr int kSlots = 16; // jobs per warp: eight in work, eight ready
+    constexpr int kSlots = 32; // jobs per warp, in work or ready
+    constexpr int kBatch = 16; // jobs fetched at once
     constexpr int kRecs = 32;  // leaf setups per warp
-    constexpr int kReps = 16;  // hit records per warp still to be made
+    constexpr int kReps = 32;  // hit records per warp still to be made
     __shared__ Bound s_rec[kLeafThreads / 32][kRecs];
     struct Slot { double t_min; int ray, tri, keep, i[kCollect], j[kCollect]; unsigned char rec[kCollect]; };
     __shared__ Slot s_job[kLeafThreads / 32][kSlots];
@@ -1363,8 +1366,9 @@ __global__ void __launch_bounds__(kLeafThreads,
     unsigned long long *fetch = round_ctr(ctr, round, 2);
     // as the walk: a round of few jobs spreads them over all warps
     const unsigned long long warps = (unsigned long long)gridDim.x * (kLeafThreads / 32);
-    const int batch = (int)min(8ull, (count + warps - 1ull) / warps);
-    int phase = (lane >> 2) < batch ? NEED : DONE;
+    const int share = (int)min(64ull, (count + warps - 1ull) / warps);
+    const int batch = share >= 4 * kBatch ? kBatch : min(8, share); // 16 of a long queue, which leaves no lane idle
+    int phase = (lane >> 2) < share ? NEED : DONE;
     unsigned long long next = 0, last = 0; // items of the queue this warp holds and has not set up
     bool more = batch > 0;                 // items may be left in the queue
     unsigned ready = 0u;                   // slots with a job set up and not yet taken
@@ -1405,7 +1409,7 @@ __global__ void __launch_bounds__(kLeafThreads,
 
     for (;;) {
         // quads without a job take one that is ready; when none is, the warp
-        // sets up the next eight of the queue, a lane per cell
+        // sets up the next ones of the queue
         unsigned need;
         while ((need = __ballot_sync(FULL, phase == NEED) & 0x11111111u) != 0u) {
             if (ready) {
@@ -1443,51 +1447,64 @@ __global__ void __launch_bounds__(kLeafThreads,
                     continue;
                 }
             }
-            // the next jobs whose cells the free setups hold: a lane per cell
-            const unsigned long long item = next + (lane >> 2);
+            // the next jobs whose cells the free setups hold, a lane per job
+            const unsigned long long item = next + lane;
+            const bool here = lane < kBatch && item < last;
             unsigned cells = 0u;
-            int jr = 0, jt = 0, li = 0, lj = 0;
-            if (item < last) {
+            int jr = 0, jt = 0;
+            if (here) {
                 const LeafJob &J = q_leaf[item];
                 cells = (unsigned)J.keep;
                 jr = J.ray;
                 jt = J.tri;
-                li = J.i[Q.sub];
-                lj = J.j[Q.sub];
             }
-            const unsigned kept = __ballot_sync(FULL, (cells >> Q.sub) & 1u);
-            const bool fits = item < last && __popc(kept & (unsigned)((16ull << Q.lead) - 1ull)) <= kRecs - __popc(recs);
-            const unsigned took = __ballot_sync(FULL, fits) & 0x11111111u;
+            int upto = __popc(cells); // cells of the jobs up to this one
+#pragma unroll 1
+            for (int x = 1; x < kBatch; x <<= 1) {
+                const int below = __shfl_up_sync(FULL, upto, x);
+                upto += lane >= x ? below : 0;
+            }
+            const bool fits = here && upto <= kRecs - __popc(recs);
+            const unsigned took = __ballot_sync(FULL, fits);
             if (!took)
                 break; // the jobs in work hold them
-            next += __popc(took);
             // the slots no quad's job is in
             const unsigned taken = __reduce_or_sync(FULL, phase == SEARCH || phase == NEWTON ? 1u << slot : 0u);
-            const int to = nth_bit(~taken, (lane >> 2));
-            unsigned mine = 0u;
+            const int to = nth_bit(~taken, lane & (kBatch - 1));
             if (fits) {
                 Slot &S = s_job[wi][to];
-                if (Q.sub == 0) {
-                    S.ray = jr;
-                    S.tri = jt;
-                    S.keep = (int)cells;
-                    if (!cells) // the filter rejected every cell of the job: the walk goes on
-                        q_out[atomicAdd(round_ctr(ctr, round, 3), 1ull)] = jr;
-                }
-                S.i[Q.sub] = li;
-                S.j[Q.sub] = lj;
-                if ((cells >> Q.sub) & 1u) {
-                    const int at = nth_bit(~recs, __popc(kept & ((1u << lane) - 1u)));
-                    S.rec[Q.sub] = (unsigned char)at;
-                    mine = 1u << at;
-                    double t0, t1;
-                    v3 O, D;
-                    const TriDev &T = tris64[jt];
-                    leaf_ray(rays, opt.ray_dtype, jr, opt.inst_xf, T.inst, O, D, t0, t1);
-                    S.t_min = t0; // the same from every lane
-                    P::setup(T, assets[T.asset], O, D, li, lj, s_rec[wi][at]);
-                }
+                S.ray = jr;
+                S.tri = jt;
+                S.keep = (int)cells;
+                if (!cells) // the filter rejected every cell of the job: the walk goes on
+                    q_out[atomicAdd(round_ctr(ctr, round, 3), 1ull)] = jr;
             }
+            // their setups, a lane per cell: the job whose cells reach past the lane
+            int job = 0;
+#pragma unroll 1
+            for (int x = kBatch / 2; x > 0; x >>= 1)
+                job += __shfl_sync(FULL, upto, job + x - 1) <= lane ? x : 0;
+            const int total = __shfl_sync(FULL, upto, __popc(took) - 1);
+            const unsigned jc = __shfl_sync(FULL, cells, job);
+            const int q = nth_bit(jc, lane - (__shfl_sync(FULL, upto, job) - __popc(jc)));
+            const int cs = __shfl_sync(FULL, to, job), cr = __shfl_sync(FULL, jr, job), ct = __shfl_sync(FULL, jt, job);
+            unsigned mine = 0u;
+            if (lane < total) {
+                Slot &S = s_job[wi][cs];
+                const LeafJob &J = q_leaf[next + job];
+                const int li = J.i[q], lj = J.j[q], at = nth_bit(~recs, lane);
+                S.i[q] = li;
+                S.j[q] = lj;
+                S.rec[q] = (unsigned char)at;
+                mine = 1u << at;
+                double t0, t1;
+                v3 O, D;
+                const TriDev &T = tris64[ct];
+                leaf_ray(rays, opt.ray_dtype, cr, opt.inst_xf, T.inst, O, D, t0, t1);
+                S.t_min = t0; // the same from every lane of the job
+                P::setup(T, assets[T.asset], O, D, li, lj, s_rec[wi][at]);
+            }
+            next += __popc(took);
             __syncwarp();
             recs |= __reduce_or_sync(FULL, mine);
             ready = __reduce_or_sync(FULL, fits && cells ? 1u << to : 0u);
