@@ -445,6 +445,7 @@ struct LeafJob
 // RayState.flags
 constexpr int kFoundInTri = 1; // a hit was taken in the triangle in progress
 constexpr int kShrunk = 2;     // the leaves of the last job shrank t_max: the cells still open are tested again
+constexpr int kExpand = 16;   // parked with the last cell taken still to expand
 constexpr int kCapped = 4;     // a triangle walk of this ray ran out of its cell-visit cap (DMAP_HIT_CAPPED)
 constexpr int kRerun = 8;      // listed for the filter's schedule (it took a crossing the filter rejects)
 
@@ -812,7 +813,8 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
         // 1. quads without work take a ray that is ready; when none is, the
         // warp fetches the next ones of the round, a lane per ray
         bool fresh = false;
-        bool enter = false; // the quad's lanes need the ray in triangle tri's frame
+        bool enter = false;  // the quad's lanes need the ray in triangle tri's frame
+        bool expand = false; // a resumed ray whose last cell's children come next
         unsigned need;
         while ((need = __ballot_sync(FULL, phase == NEED) & 0x11111111u) != 0u) {
             if (TREE && __popc(need) < pick_quads && __any_sync(FULL, phase == WALK || phase == TOP || phase == LEAF))
@@ -907,7 +909,8 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                     tmax_f = __double2float_ru(t_max);
                     enter = true;
                     stale = (flags & kShrunk) ? ~0u : 0u;
-                    flags &= ~kShrunk;
+                    expand = (flags & kExpand) != 0;
+                    flags &= ~(kShrunk | kExpand);
                     guard = 0;
                     nl = 0;
                     phase = WALK;
@@ -1125,7 +1128,7 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
         unsigned cells = 15u;
         if (phase == WALK) {
             const int root_level = tris32[tri].root_level;
-            if (test) {
+            if (roots) {
                 tl = root_level;
                 cells = (1u << tris32[tri].n_roots) - 1u;
                 if (DEEP && tl > 31) { // beyond the bits of the open groups
@@ -1136,16 +1139,28 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                     test = false;
                 }
             }
+            if (expand) {
+                tl = cur.level - 1;
+                pi = cur.i;
+                pj = cur.j;
+                test = true;
+            }
             bool parking = false;
             while (!test && phase == WALK && !parking) {
                 if (!todo.any()) {
                     // the end of the triangle's walk
                     if (ST) {
-                        const int left = dom.count();
+                        // with leaves collected, at most the tests before a park
+                        int left = dom.count();
+                        if (nl > 0 && since + left > DMAP_STALE_CAP)
+                            left = DMAP_STALE_CAP + 1 - since;
                         stl[DMAP_ST_NODE] += left;
                         nah += left;
+                        for (; left > 0; --left)
+                            dom.clear_bit(dom.first());
+                    } else {
+                        dom = {0ull, 0ull};
                     }
-                    dom = {0ull, 0ull};
                     if (!INLINE_LEAF && nl > 0) {
                         // the collected leaves decide this triangle's t_max before the next one
                         parking = true;
@@ -1198,10 +1213,6 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                     nah += n_in;
                 }
                 dom.clear_upto(p);
-                if (l > 0 && nl > 0 && since > DMAP_STALE_CAP) {
-                    parking = true; // the cell is taken (and its group tested) again after the resume
-                    break;
-                }
                 todo.clear_bit(p);
                 const TriDev32 &T = tris32[tri];
                 cur.level = l;
@@ -1212,6 +1223,11 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                     pi = cur.i;
                     pj = cur.j;
                     test = true;
+                    if (!INLINE_LEAF && nl > 0 && since > DMAP_STALE_CAP) {
+                        flags |= kExpand; // its children are tested after the resume
+                        parking = true;
+                        test = false;
+                    }
                     break;
                 }
                 if (ST) {
