@@ -404,6 +404,19 @@ struct CellBits
     }
 };
 
+// The cells of the open groups that come after cell (l, i, j) in walk order:
+// its later siblings and those of the cells above it. The walk counts a
+// group's cells when it tests them, all at once; less those still ahead this
+// is what the one-cell walk has visited, which opt.guard_cap bounds.
+__device__ __noinline__ int cells_ahead(const TriDev32 &T, int l, int i, int j, int si, int sj)
+{
+    const int up = T.root_level - l, m = (int)((1u << up) - 1u);
+    int k = 0;
+    while (k + 1 < T.n_roots && (T.roots_i[k] != i >> up || T.roots_j[k] != j >> up))
+        ++k;
+    return T.n_roots - 1 - k + 3 * up - 2 * __popc((i ^ -si) & m) - __popc((j ^ -sj) & m);
+}
+
 // A parked walk: the ray's position in ObjectIntersector's triangle loop and
 // in DisplacedIntersector's walk (the cell last taken and the open groups'
 // bits), its current t_max and result, its candidate mask and the counters
@@ -527,7 +540,7 @@ __device__ __noinline__ double quad_leaf(const TriDev32 &T32, const TriDev &T, c
         if (e.depth + 1 < lq::kDepth)
             lq::push_children<P>(Q, c, e.depth + 1, stack, sp);
         else if (c.n > 0 && lq::newton_children<P, ST>(Q, c, T, g, L, ray_of, t_min, t_max, i, j, opt.polish_cond,
-                                                       opt.mode == 1, iters, on_root))
+                                                       opt.mode == 1 && !opt.op_mask, iters, on_root))
             break;
     } while (lq::pop<P>(stack, sp, t_max, e));
     if (mine == t_max && t_max < t_start) {
@@ -911,7 +924,6 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                     stale = (flags & kShrunk) ? ~0u : 0u;
                     expand = (flags & kExpand) != 0;
                     flags &= ~(kShrunk | kExpand);
-                    guard = 0;
                     nl = 0;
                     phase = WALK;
                 }
@@ -1119,6 +1131,8 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                 t1 = fmaxf(x.t1, tmin_f);
             }
             enter_frame(T, slots[slot].o, slots[slot].d, far_bound(t1));
+            if (!test)
+                guard = cells_ahead(T, cur.level, cur.i, cur.j, si, sj);
         }
         __syncwarp();
 
@@ -1149,6 +1163,10 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
             while (!test && phase == WALK && !parking) {
                 if (!todo.any()) {
                     // the end of the triangle's walk
+                    if (guard > opt.guard_cap) { // a finite tree: the cap guards corrupt records
+                        atomicOr(status, dmapdev::kStatusCapped);
+                        flags |= kCapped;
+                    }
                     if (ST) {
                         // with leaves collected, at most the tests before a park
                         int left = dom.count();
@@ -1218,6 +1236,12 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                 cur.level = l;
                 cur.i = at_root ? T.roots_i[k] : 2 * pi + ((k >> 1) ^ si);
                 cur.j = at_root ? T.roots_j[k] : 2 * pj + ((k & 1) ^ sj);
+                if (guard > opt.guard_cap &&
+                    guard - cells_ahead(T, cur.level, cur.i, cur.j, si, sj) > opt.guard_cap) {
+                    todo = {0ull, 0ull}; // gives up before this cell
+                    dom = {0ull, 0ull};
+                    continue;
+                }
                 if (l > 0) {
                     tl = l - 1;
                     pi = cur.i;
@@ -1305,12 +1329,6 @@ __global__ void __launch_bounds__(128, INLINE_LEAF ? DMAP_DRAIN_MIN_BLOCKS
                 if (roots)
                     cur = {tl + 1, 0, 0};
                 guard += __popc(cells);
-                if (guard > opt.guard_cap) { // a finite tree: the cap guards corrupt records
-                    atomicOr(status, dmapdev::kStatusCapped);
-                    flags |= kCapped;
-                    todo = {0ull, 0ull};
-                    dom = {0ull, 0ull};
-                }
             }
         }
     }
@@ -1606,7 +1624,7 @@ __global__ void __launch_bounds__(kLeafThreads,
                 const double t_old = t_max;
                 phase = SEARCH;
                 if (lq::newton_children<P, ST>(Q, c, T, assets[T.asset], s_rec[wi][rec], ray_of, t_min, t_max, ci, cj, opt.polish_cond,
-                                               opt.mode == 1, iters, on_root)) {
+                                               opt.mode == 1 && !opt.op_mask, iters, on_root)) {
                     // occlusion: any hit answers the query
                     answered = true;
                     sp = 0;

@@ -4,6 +4,8 @@ triangle counts around the 32 boxes of a ballot and the last one of the
 candidate mask; charts whose root level is past the 64 bits of open groups
 (the wider bits), mirrored and off the cell lattice. Every record equals the
 oracle's bit for bit with the FP64 leaf, in both orders."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -95,3 +97,26 @@ def test_leaf_rounds_agree(ctx, oracle, n, leaf):
     for rounds in (0, 1, 2):
         o = dev.intersect(rays, dm.TraversalOptions(rounds=rounds, leaf_precision=leaf, mode="occluded"), np.float64)
         assert np.array_equal(o["tri"] >= 0, base["tri"] >= 0)
+
+
+@pytest.mark.parametrize("cap", [1, 2, 3, 5, 9, 14, 22, 35])
+def test_visit_cap_counts_cells_in_walk_order(ctx, oracle, cap):
+    """A group is tested at once; the cap counts the cells the one-cell walk
+    visits. The simple schedule counts them per root (at most 4 a triangle):
+    what runs out there runs out here, what does not lasts here at 4 x cap."""
+    sc = helpers.small_sphere(32)
+    cpu, dev = py_oracle.CpuScene(oracle, sc), dm.Scene.from_synthetic(ctx, sc)
+    rays = np.concatenate([helpers.near_surface_rays(cpu, 1500), helpers.aimed_rays(cpu, 500)[0]])
+    rays = np.ascontiguousarray(rays, np.float32)
+
+    def capped(schedule, c):
+        o = dm.TraversalOptions(schedule=schedule, rounds=0, node_visit_cap=c, leaf_precision="f64").c()
+        hits = np.empty(len(rays), dm.HIT64)
+        st = dm.lib().dmap_intersect_host(dev.h, rays.ctypes.data, dm.F32, len(rays), C.byref(o), hits.ctypes.data,
+                                          dm.F64, None)
+        flags = (hits["flags"] & dm.HIT_CAPPED) != 0
+        assert st == (6 if flags.any() else 0)  # DMAP_ERR_LIMIT
+        return flags
+
+    simple, wave, wide = capped("simple", cap), capped("wavefront", cap), capped("wavefront", 4 * cap)
+    assert simple.any() and not (simple & ~wave).any() and not (wide & ~simple).any()
