@@ -407,8 +407,9 @@ struct CellBits
 // The cells of the open groups that come after cell (l, i, j) in walk order:
 // its later siblings and those of the cells above it. The walk counts a
 // group's cells when it tests them, all at once; less those still ahead this
-// is what the one-cell walk has visited, which opt.guard_cap bounds.
-__device__ __noinline__ int cells_ahead(const TriDev32 &T, int l, int i, int j, int si, int sj)
+// is what the one-cell walk has visited, which opt.guard_cap bounds. Called
+// out of line it cost the walk 1% (14.06 -> 14.18 ms at 2.80M rays).
+__device__ __forceinline__ int cells_ahead(const TriDev32 &T, int l, int i, int j, int si, int sj)
 {
     const int up = T.root_level - l, m = (int)((1u << up) - 1u);
     int k = 0;
