@@ -540,9 +540,8 @@ __device__ __noinline__ double quad_leaf(const TriDev32 &T32, const TriDev &T, c
             subs += 4;
         if (e.depth + 1 < lq::kDepth)
             lq::push_children<P>(Q, c, e.depth + 1, stack, sp);
-        else if (c.n > 0 && lq::newton_children<P, ST>(Q, c, T, g, L, ray_of, t_min, t_max, i, j, opt.polish_cond,
-                                                       opt.mode == 1 && !opt.op_mask, iters, on_root))
-            break;
+        else if (c.n > 0) // the leaf's nearest root, in an occlusion query too: the simple schedule's record
+            lq::newton_children<P, ST>(Q, c, T, g, L, ray_of, t_min, t_max, i, j, opt.polish_cond, false, iters, on_root);
     } while (lq::pop<P>(stack, sp, t_max, e));
     if (mine == t_max && t_max < t_start) {
         d64::hit64 h;
