@@ -1623,9 +1623,10 @@ __global__ void __launch_bounds__(kLeafThreads,
                 };
                 const double t_old = t_max;
                 phase = SEARCH;
-                if (lq::newton_children<P, ST>(Q, c, T, assets[T.asset], s_rec[wi][rec], ray_of, t_min, t_max, ci, cj, opt.polish_cond,
-                                               opt.mode == 1 && !opt.op_mask, iters, on_root)) {
-                    // occlusion: any hit answers the query
+                if (lq::newton_children<P, ST>(Q, c, T, assets[T.asset], s_rec[wi][rec], ray_of, t_min, t_max, ci, cj,
+                                               opt.polish_cond, opt.mode == 1, iters, on_root)) {
+                    // occlusion: any hit answers the query (one that an opacity
+                    // mask rejects hands the ray to the filter's schedule)
                     answered = true;
                     sp = 0;
                 }
