@@ -27,7 +27,7 @@ cudaError_t walk_round(const Args &a, const int *q_in, int round, cudaStream_t s
     cudaError_t e = cudaSuccess;
     auto run = [&](auto *kernel, int64_t *stats) {
         if (bytes > 32256)
-            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+            e = allow_entries(kernel);
         if (e == cudaSuccess)
             kernel<<<a.grid, 128, bytes, stream>>>(a.t32, a.t64, a.n_tri, a.assets, a.rays, a.n, a.opt, a.hits, stats,
                                                    states, q_in, round, leaves, a.counters, a.status, a.rerun);

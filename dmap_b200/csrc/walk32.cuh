@@ -1640,6 +1640,15 @@ __global__ void __launch_bounds__(kLeafThreads,
 
 // Dynamic shared memory of the walk: the candidates' box entries.
 size_t entry_bytes(int n_tri) { return n_tri > 32 * kMaskWords ? 0 : (size_t)(n_tri + 3) / 4 * 128 * sizeof(float); }
+// The opt-in to more of it than needs none, for the largest scene that takes
+// the mask whatever the scene at hand: the attribute is the kernel's, and
+// another thread's launch over a larger scene may stand between this thread's
+// opt-in and its launch.
+template <class Kernel>
+cudaError_t allow_entries(Kernel *kernel)
+{
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)entry_bytes(32 * kMaskWords));
+}
 
 int sm_count()
 {
