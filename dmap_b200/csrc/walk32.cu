@@ -21,13 +21,10 @@ cudaError_t walk_round(const Args &a, const int *q_in, int round, cudaStream_t s
     const bool nearest = a.opt.order == 1, tree = a.n_tri > 32 * kMaskWords;
     RayState *states = static_cast<RayState *>(a.states);
     LeafJob *leaves = static_cast<LeafJob *>(a.leaves);
-    // the entries of more than 252 triangles pass the 48 KB of shared memory
-    // that need no opt-in
     const size_t bytes = entry_bytes(a.n_tri);
     cudaError_t e = cudaSuccess;
     auto run = [&](auto *kernel, int64_t *stats) {
-        if (bytes > 32256)
-            e = allow_entries(kernel);
+        e = bytes > 0 ? allow_entries(kernel) : cudaSuccess;
         if (e == cudaSuccess)
             kernel<<<a.grid, 128, bytes, stream>>>(a.t32, a.t64, a.n_tri, a.assets, a.rays, a.n, a.opt, a.hits, stats,
                                                    states, q_in, round, leaves, a.counters, a.status, a.rerun);
