@@ -76,8 +76,6 @@ struct alignas(128) TriDev32
     float qerr;    // 2 G of the same sum of |N|^2's terms
     float udm[3];  // ud less the domain test's rounding over the footprint's cells
     int log2n;     // the asset's pyramid: 2^log2n leaf cells per side
-    float perr[3]; // 2 G (X, Y, 0): the base point's roundings
-    float pad1;
     const float *pyr32;
     int root_level, n_roots, asset, pad2;
     int roots_i[4], roots_j[4];

@@ -301,7 +301,7 @@ __device__ void derive32(const TriDev &T, const AssetDev &g, TriDev32 &S)
     S.root_level = T.root_level;
     S.n_roots = T.n_roots;
     S.asset = T.asset;
-    S.pad0 = S.pad1 = 0.0f;
+    S.pad0 = 0.0f;
     S.pad2 = 0;
     for (int k = 0; k < 4; ++k) {
         S.roots_i[k] = T.roots_i[k];
@@ -331,9 +331,6 @@ __device__ void derive32(const TriDev &T, const AssetDev &g, TriDev32 &S)
     const double q = fabs(dot3(m0, m0)) + 2.0 * (X * fabs(dot3(m0, Mu)) + Y * fabs(dot3(m0, Mv))) +
                      (X * X * dot3(Mu, Mu) + Y * Y * dot3(Mv, Mv)) + 2.0 * X * Y * fabs(dot3(Mu, Mv));
     S.qerr = fup(2.0 * G * q * (1.0 + G));
-    S.perr[0] = fup(2.0 * G * X);
-    S.perr[1] = fup(2.0 * G * Y);
-    S.perr[2] = 0.0f;
     // a footprint's cell reaches at most two root widths past the domain
     const double w = cell_width(g, T.root_level);
     for (int k = 0; k < 3; ++k) {

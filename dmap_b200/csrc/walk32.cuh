@@ -97,7 +97,7 @@ __device__ __forceinline__ void tangent_row(const TriDev32 &T, int a, const doub
     const float um = fmaxf(fmaxf(fabsf((float)u0), fabsf((float)u1)), fabsf((float)u2));
     const float dm = fmaxf(fmaxf(fabsf((float)d0), fabsf((float)d1)), fabsf((float)d2));
     const float sum = ru_mul(__double2float_ru(fabs(A0) + fabs(A1) + fabs(A2)), ru_fma(t_far, dm, um));
-    e = ru_add(ru_fma(0x1p-22f, ru_fma(t_far, fabsf(rd), fabsf(ro)), ru_mul(0x1.1p-40f, sum)), T.perr[a]);
+    e = ru_fma(0x1p-22f, ru_fma(t_far, fabsf(rd), fabsf(ro)), ru_mul(0x1.1p-40f, sum));
 }
 
 __device__ __forceinline__ void tangent_ray(const TriDev32 &T, const double *o, const double *d, float t_far,
