@@ -160,7 +160,6 @@ dmap_status dmap_asset_create(dmap_context *ctx, const void *values_host, dmap_d
     d.nodes = a->nodes;
     d.pyr64 = keep64 ? a->pyr64 : nullptr;
     d.pyr32 = a->pyr32;
-    double *const levels64 = a->pyr64 - 8 * first64; // indexed by cell from level 0
 
     // TMA descriptor over the node grid: a (T+1) x box_w tile per CTA.
     EncodeTiledFn enc = encode_tiled();
@@ -190,8 +189,9 @@ dmap_status dmap_asset_create(dmap_context *ctx, const void *values_host, dmap_d
     if (direct && (e = cudaMalloc(&hull, ((size_t)cells + 32768) * 32)) != cudaSuccess)
         return cleanup(cuda_fail(ctx, e, "dmap_asset_create: cudaMalloc"));
     cudaEventRecord(ev[0], ctx->stream);
-    e = direct ? dmapk::launch_pyramid_direct(d, levels64, a->pyr32, hull, ctx->stream, keep64)
-               : dmapk::launch_pyramid(&tmap, d, T, levels64, a->pyr32, ctx->status_dev, ctx->stream, keep64);
+    e = direct ? dmapk::launch_pyramid_direct(d, a->pyr64, a->pyr32, hull, ctx->stream, keep64)
+               : dmapk::launch_pyramid(&tmap, d, T, a->pyr64, a->pyr32, ctx->status_dev, ctx->stream, keep64,
+                                       (size_t)first64);
     cudaEventRecord(ev[1], ctx->stream);
     if (e != cudaSuccess) {
         cudaEventDestroy(ev[0]);

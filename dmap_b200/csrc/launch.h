@@ -75,13 +75,15 @@ int walk32_launches(const QueryOpts &opt);
 // levels without the offset into pyr64 and the outward-rounded FP32 levels
 // with it into pyr32.
 // all64: write every FP64 level (the FP64 pyramid is kept); otherwise only
-// the levels the fold launches read back, which are scratch.
+// the levels the fold launches read back, which are scratch. pyr64 starts at
+// cell first64: without all64 nothing below the first tile's top is written.
 cudaError_t launch_pyramid(const void *tmap, const dmapdev::AssetDev &a, int tile, double *pyr64, float *pyr32,
-                           unsigned *status, cudaStream_t stream, bool all64 = true);
+                           unsigned *status, cudaStream_t stream, bool all64 = true, size_t first64 = 0);
 
 // The Direct build (taylor_pyramid.cpp:151-202): every level from the node
 // grid. hull_scratch holds 32 bytes per pyramid cell plus 32768 x 32 bytes
-// of partial hulls; 2 or 3 launches per level (direct_launches).
+// of partial hulls; 2 or 3 launches per level (direct_launches). pyr64 is
+// written with all64 only.
 int direct_launches(int n_leaf);
 cudaError_t launch_pyramid_direct(const dmapdev::AssetDev &a, double *pyr64, float *pyr32, void *hull_scratch,
                                   cudaStream_t stream, bool all64);
