@@ -23,7 +23,6 @@ __device__ __forceinline__ float rd_add(float x, float y) { return __fadd_rd(x, 
 __device__ __forceinline__ float ru_mul(float x, float y) { return __fmul_ru(x, y); }
 __device__ __forceinline__ float rd_mul(float x, float y) { return __fmul_rd(x, y); }
 __device__ __forceinline__ float ru_fma(float x, float y, float z) { return __fmaf_ru(x, y, z); }
-__device__ __forceinline__ float mag3(float x, float y, float z) { return ru_add(ru_add(fabsf(x), fabsf(y)), fabsf(z)); }
 // 2^e exactly, -126 <= e <= 127
 __device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }
 
@@ -262,7 +261,7 @@ __device__ __forceinline__ float quot_dn(float a, float b)
 // <= slab_max_level the slab, both enclosing their double counterparts. Its
 // roundings are bounded by constants of the triangle where a bound over the
 // domain is as good as one at the cell (a box coordinate took 52 operations
-// with every magnitude summed, 33 so: walk rounds of 2.80M rays on 96 x
+// with every magnitude summed, 33 to 35 so: walk rounds of 2.80M rays on 96 x
 // 2048^2 maps 14.6 -> 13.6 ms).
 __device__ __forceinline__ bool node_test32(const Walk32 &T, const float *pyr32, const Ray32 &r, int level, int i,
                                             int j, float t_min, float t_max, int bound, int slab_max_level)

@@ -97,21 +97,9 @@ __device__ inline void root_record(const TriDev &T, const AssetDev &g, double t,
     hit.j = j;
 }
 
-// What a leaf's setup computes (208 bytes, thirteen 16-byte words), and with
-// the texel and the ray's origin, which follow from the cell and the ray.
-struct alignas(16) leafrec { double h00, h10, h01, h11; af3 N_hat; v3 dn, d1, d2; double d_len; };
-static_assert(sizeof(leafrec) == 208, "leaf record");
-struct leafbound : leafrec
-{
-    v2 lo;
-    double w;
-    v3 o;
-    __device__ __forceinline__ void place(const AssetDev &g, int64_t i, int64_t j)
-    {
-        w = cell_width(g, 0);
-        lo = {i * w, j * w};
-    }
-};
+// What a leaf's setup computes: the texel's corner heights, its normal form and
+// the ray's plane basis; the texel and the ray's origin.
+struct alignas(16) leafbound { double h00, h10, h01, h11; af3 N_hat; v3 dn, d1, d2; double d_len; v2 lo; double w; v3 o; };
 
 __device__ __forceinline__ af restricted(af f, double a, double b, double rho) // :72-76
 {
@@ -151,7 +139,8 @@ struct leafent { double a, b, t_lo; int depth; };
 // and the ray's plane basis.
 __device__ inline void leaf_setup(const TriDev &T, const AssetDev &g, v3 o, v3 d, int64_t i, int64_t j, leafbound &L)
 {
-    L.place(g, i, j);
+    L.w = cell_width(g, 0);
+    L.lo = {i * L.w, j * L.w};
     double hc[4];
 #pragma unroll 1
     for (int q = 0; q < 4; ++q)

@@ -43,9 +43,8 @@ using namespace d64;
 
 constexpr float kG2 = 2.0f * d32::G; // margin factor of the bound's terms
 
-// What the setup computes (192 bytes: kept as twelve 16-byte words between
-// the kernel that sets leaves up and the one that searches them).
-struct alignas(16) Rec32
+// What a leaf's setup computes, for its search and its roots.
+struct alignas(16) Leaf32
 {
     double Q3, inv_dlen;  // dn . (X0 - o) and 1 / |d|, in double
     float q0, q1;         // d1 . (X0 - o), d2 . (X0 - o)
@@ -58,25 +57,14 @@ struct alignas(16) Rec32
     float Mcu, Mcv, Muu, Muv, Mvv, Mcc, Mlc; // M0 . Mu w/2, ..., |M0|^2, |M0|
     float hmid, d00, ha, hb, tw; // h(a, b) = hmid + d00 + ha a + hb b + tw a b
     float tol2;           // Newton acceptance: residual^2 below this
-};
-static_assert(sizeof(Rec32) == 192, "leaf record");
-
-struct Leaf32 : Rec32
-{
     double lo_s, lo_t, w; // the texel in chart coordinates
-    __device__ __forceinline__ void place(const AssetDev &g, int64_t i, int64_t j)
-    {
-        w = cell_width(g, 0);
-        lo_s = i * w;
-        lo_t = j * w;
-    }
 };
 
 // intersect_newton's setup (:239-264) and the leaf's FP32 terms.
 __device__ inline void leaf_setup32(const TriDev &T, const AssetDev &g, v3 o, v3 d, int64_t i, int64_t j, Leaf32 &L)
 {
-    L.place(g, i, j);
-    const double w = L.w, los = L.lo_s, lot = L.lo_t;
+    const double w = cell_width(g, 0), los = i * w, lot = j * w;
+    L.lo_s = los, L.lo_t = lot, L.w = w;
     double hc[4]; // one copy of the lookup's code: the leaf kernels wait on instruction fetch
 #pragma unroll 1
     for (int q = 0; q < 4; ++q)

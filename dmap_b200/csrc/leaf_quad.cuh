@@ -38,18 +38,11 @@ struct P32
 {
     using Real = float;
     using Bound = l32::Leaf32;
-    using Rec = l32::Rec32;
     using Root = l32::Root32;
     struct Ent { float a, b, t_lo; int depth; };
     static __device__ __forceinline__ void setup(const TriDev &T, const AssetDev &g, v3 o, v3 d, int i, int j, Bound &L)
     {
         l32::leaf_setup32_shared(T, g, o, d, i, j, L);
-    }
-    // a stored setup's leaf, for the cell and the ray it was made for
-    template <class Ray>
-    static __device__ __forceinline__ void place(const AssetDev &g, const Ray &, int i, int j, Bound &L)
-    {
-        L.place(g, i, j);
     }
     static __device__ __forceinline__ bool bound(const TriDev32 &T32, const TriDev &, const Bound &L, float a, float b,
                                                  float rho, double t_min, double t_max, float &t_lo)
@@ -75,19 +68,11 @@ struct P64
 {
     using Real = double;
     using Bound = d64::leafbound;
-    using Rec = d64::leafrec;
     using Root = hit64;
     struct Ent { double t_lo; float a, b; int depth; }; // a, b: multiples of 2^-6, exact
     static __device__ __forceinline__ void setup(const TriDev &T, const AssetDev &g, v3 o, v3 d, int i, int j, Bound &L)
     {
         d64::leaf_setup_shared(T, g, o, d, i, j, L);
-    }
-    template <class Ray>
-    static __device__ __forceinline__ void place(const AssetDev &g, const Ray &ray, int i, int j, Bound &L)
-    {
-        L.place(g, i, j);
-        v3 d;
-        ray(L.o, d);
     }
     static __device__ __forceinline__ bool bound(const TriDev32 &, const TriDev &T, const Bound &L, float a, float b,
                                                  float rho, double t_min, double t_max, double &t_lo)

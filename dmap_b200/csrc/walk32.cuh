@@ -25,12 +25,12 @@
 //  - wavefront (default): rounds of two persistent kernels. The walk kernel
 //    gives each ray four lanes, which test the four cells of a sibling group
 //    together: a ray that reaches leaves writes a leaf job, parks its walk
-//    state and its lanes take the next ray; the leaf kernel runs the parked leaves, one job per lane, each
-//    lane taking the next job when its own is done, and queues their rays
-//    to resume. After `rounds` rounds a last walk runs the few
-//    remaining rays with their leaves inline. Every ray still visits its
-//    cells in the reference's order with the reference's t_max, so its hit
-//    is the one the simple schedule finds.
+//    state and its lanes take the next ray; the leaf kernel runs the parked
+//    leaves, a job per quad of lanes, and queues their rays to resume.
+//    After `rounds` rounds a last walk runs the few remaining rays with
+//    their leaves inline. Every ray still visits its cells in the
+//    reference's order with the reference's t_max, so its hit is the one
+//    the simple schedule finds.
 //
 // The kernels live in this header and are instantiated by two translation
 // units (walk32_launch.h lists which launches each one owns):
